@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -15,14 +16,91 @@ int fail(int code, const std::string& msg) {
 }
 
 namespace {
-// RAII device scratch for the host-pointer convenience entry points
+// Device scratch of the operator entry points, kept between calls: cudaMalloc + cudaFree (which waits for the device and
+// unmaps) cost 0.6-3 ms per call of a 37-row matmul whose kernels take 20 us. A buffer belongs to one call from alloc()
+// to the end of its scope, which every entry point reaches after its own synchronize, so calls on other threads and
+// streams never meet in one. Bounded: at most SCRATCH_KEEP idle buffers and SCRATCH_BYTES in all stay per device; the
+// rest, and everything when the last weight of the device goes or an allocation fails, is given back to the driver.
+constexpr size_t SCRATCH_KEEP = 6, SCRATCH_BYTES = size_t(256) << 20;
+struct Scratch {
+    struct Buf { void* p; size_t bytes; };
+    std::mutex mu;
+    std::vector<Buf> idle;
+    size_t idle_bytes = 0;
+    int weights = 0;  // live weights made by elb_weight_create
+
+    void* take(size_t n, size_t* got) {
+        std::lock_guard<std::mutex> lock(mu);
+        size_t best = idle.size();
+        for (size_t i = 0; i < idle.size(); ++i)  // the smallest that fits, unless it would be mostly idle space
+            if (idle[i].bytes >= n && idle[i].bytes / 8 <= n + 65536 && (best == idle.size() || idle[i].bytes < idle[best].bytes)) best = i;
+        if (best == idle.size()) return nullptr;
+        void* p = idle[best].p;
+        *got = idle[best].bytes;
+        idle_bytes -= idle[best].bytes;
+        idle.erase(idle.begin() + long(best));
+        return p;
+    }
+    void give(void* p, size_t bytes) {
+        std::vector<Buf> out;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (weights > 0 && bytes <= SCRATCH_BYTES) {
+                idle.push_back({p, bytes});
+                idle_bytes += bytes;
+                while (idle.size() > SCRATCH_KEEP || idle_bytes > SCRATCH_BYTES) {  // the oldest goes first
+                    out.push_back(idle.front());
+                    idle_bytes -= idle.front().bytes;
+                    idle.erase(idle.begin());
+                }
+            } else {
+                out.push_back({p, bytes});
+            }
+        }
+        for (const Buf& b : out) cudaFree(b.p);
+    }
+    void release() {
+        std::vector<Buf> out;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            out.swap(idle);
+            idle_bytes = 0;
+        }
+        for (const Buf& b : out) cudaFree(b.p);
+    }
+    void count(int d) {
+        bool last = false;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            weights += d;
+            last = weights == 0;
+        }
+        if (last) release();
+    }
+};
+Scratch& scratch_of(int device) {
+    static Scratch* const pools = new Scratch[64];  // never destroyed: a weight may outlive the library's static objects
+    return pools[device >= 0 && device < 64 ? device : 0];
+}
 struct Dev {
     void* p = nullptr;
-    ~Dev() { if (p) cudaFree(p); }
-    int alloc(size_t n) {
-        if (cudaMalloc(&p, std::max<size_t>(n, 16)) != cudaSuccess) {
+    size_t bytes = 0;
+    int device = 0;
+    ~Dev() { if (p) scratch_of(device).give(p, bytes); }
+    int alloc(size_t n) {  // on the current device
+        ELB_CUDA(cudaGetDevice(&device));
+        n = (std::max<size_t>(n, 16) + 511) / 512 * 512;
+        p = scratch_of(device).take(n, &bytes);
+        if (p) return ELB_OK;
+        bytes = n;
+        if (cudaMalloc(&p, n) != cudaSuccess) {
             cudaGetLastError();
-            return fail(ELB_ERR_MEMORY, "out of device memory");
+            scratch_of(device).release();
+            if (cudaMalloc(&p, n) != cudaSuccess) {
+                cudaGetLastError();
+                p = nullptr;
+                return fail(ELB_ERR_MEMORY, "out of device memory");
+            }
         }
         return ELB_OK;
     }
@@ -102,10 +180,16 @@ int elb_weight_create(int device, int ggml_type, int64_t rows, int64_t n, const 
     ELB_TRY(weight_create(device, ggml_type, rows, n, bytes, nbytes, flags, &w));
     const int rc = gemv_prepare(w);
     if (rc != ELB_OK) { weight_destroy(w); return rc; }
+    scratch_of(device).count(1);
     *out = reinterpret_cast<elb_weight*>(w);
     return ELB_OK;
 }
-void elb_weight_destroy(elb_weight* w) { weight_destroy(W(w)); }
+void elb_weight_destroy(elb_weight* w) {
+    if (!w) return;
+    const int device = W(w)->device;
+    weight_destroy(W(w));
+    scratch_of(device).count(-1);
+}
 int64_t elb_weight_rows(const elb_weight* w) { return W(w)->rows; }
 int64_t elb_weight_cols(const elb_weight* w) { return W(w)->n; }
 size_t elb_weight_device_bytes(const elb_weight* w) { return W(w)->tiled_bytes; }
@@ -137,6 +221,7 @@ static int matvec_on(const Weight* w, const float* d_x, float* d_y, int nl, cuda
     if (w->type != ELB_F16) {
         ELB_TRY(prep_limbs_launch(d_x, int(w->n), nullptr, 0.f, nl == 0 ? 4 : nl, w->xlimbs, w->xinv, false, s));
         a.limbs = w->xlimbs; a.inv_scale = w->xinv;
+        a.pdl = true;  // the matvec fills its weight rings while the split runs
     }
     return gemv_launch(w, a, s);
 }

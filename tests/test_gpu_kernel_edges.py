@@ -1,0 +1,74 @@
+"""Kernels and dispatch branches at the sizes where they can go wrong (edges of tiles, remainders, smallest and largest
+of a range), through the public entry points, against the CPU oracle or the host's own arithmetic."""
+import numpy as np
+import pytest
+
+import oracle_lib as ol
+from exactinfer_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def elb():
+    import exactinfer_b200 as e
+    ok, why = e.cuda_available()
+    assert ok, f"CUDA path unavailable: {why}"
+    return e
+
+
+# vectors shorter than the split kernel's cluster, a ragged cut over it, and one past what its registers hold
+@pytest.mark.parametrize("n", (256, 256 * 9, 32768, 32768 + 256))
+def test_split_of_one_vector_over_a_cluster(elb, n):
+    rng = np.random.default_rng(n)
+    wb = synth.rand_weight(rng, synth.Q4_K, 16, n)
+    x = rng.normal(size=n).astype(np.float32)
+    w = elb.Weight(synth.Q4_K, 16, n, wb)
+    P, I, J = w.limb_sums(x, 4)
+    limbs, _, _ = ol.split_limbs(x, 4)
+    assert np.array_equal(P, ol.limb_partials(synth.Q4_K, 16, n, wb, limbs))
+    wI, wJ = ol.limb_block_sums(synth.Q4_K, 16, n, wb, limbs)
+    assert np.array_equal(I, wI) and np.array_equal(J, wJ)
+
+
+def test_operator_scratch_is_reused_and_given_back(elb):
+    """The scratch of the operator calls is kept between calls and freed with the last weight."""
+    import ctypes as C
+    from exactinfer_b200 import capi
+
+    def free():
+        f, t = C.c_size_t(), C.c_size_t()
+        capi.check(capi.lib().elb_device_mem_info(0, C.byref(f), C.byref(t)))
+        return f.value
+
+    rng = np.random.default_rng(1)
+    before = free()
+    w = elb.Weight(synth.Q8_0, 64, 256, synth.rand_weight(rng, synth.Q8_0, 64, 256), planes=True)
+    x = rng.normal(size=(40, 256)).astype(np.float32)
+    y = w.matmul(x)
+    held = free()
+    for b in (40, 3, 17, 40):
+        assert np.array_equal(w.matmul(x[:b]).shape, (b, 64))
+    assert np.array_equal(w.matmul(x), y) and free() == held
+    w.close()
+    assert free() >= before
+
+
+# vocabularies below, at and just past a chunk of the reduction (2560 logits), and of several chunks
+@pytest.mark.parametrize("vocab", (64, 2559, 2560, 2561, 7681))
+def test_top_tokens_at_chunk_edges(elb, vocab):
+    spec = synth.Spec(name="small", n_layer=1, n_embd=256, n_ff=512, n_head=4, n_head_kv=2, n_vocab=vocab, layout="q8_0",
+                      head_sigma=1e-4)
+    tens = list(synth.generate(spec, vocab))
+    role, layer, t, rows, n, emb = tens[0]
+    emb[vocab // 2:vocab // 2 + 20] = emb[0]  # equal rows of the tied head: equal logits, the lower id comes first
+    gpu = elb.Backend(spec, tens, 40, n_seq=3)
+    toks = np.array([5, 9, 11], np.int32)
+    for k in (1, 33, 64):
+        full = gpu.eval_batch(toks, [0, 1, 2], [0, 0, 0])
+        ids, vals, lse = gpu.eval_batch_top(toks, [0, 1, 2], [0, 0, 0], k=k)
+        for r in range(3):
+            order = np.lexsort((np.arange(vocab), -full[r].astype(np.float64)))[:k]
+            assert np.array_equal(ids[r], order) and np.array_equal(vals[r], full[r][order])
+            assert abs(lse[r] - ol.logsumexp(full[r])) <= 1e-12 * max(1.0, abs(lse[r]))
+    gpu.close()
