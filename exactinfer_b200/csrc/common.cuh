@@ -289,8 +289,9 @@ int rmsnorm_launch(float* out, const float* x, const float* w, int n, float eps,
 // TOP_MAXK int32 ids, then TOP_MAXK floats
 constexpr int TOP_MAXK = 64;
 constexpr size_t TOP_BYTES = 8 + size_t(TOP_MAXK) * 8;
-int logits_top_launch(const float* logits, int n, int k, uint8_t* out, cudaStream_t s, const uint32_t* d_allowed = nullptr);
-int logits_top_rows_launch(const float* logits, int n, int64_t ld, int rows, int k, uint8_t* out, cudaStream_t s);
+size_t logits_top_scratch_bytes(int n, int rows);
+int logits_top_launch(const float* logits, int n, int64_t ld, int rows, int k, uint8_t* out, void* scratch, int scratch_rows,
+                      cudaStream_t s, const uint32_t* d_allowed = nullptr);
 
 
 }  // namespace elb

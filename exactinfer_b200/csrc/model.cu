@@ -103,6 +103,7 @@ struct Model {
     uint8_t* top_dev = nullptr;      // device-side logits post-processing: lse, ids, logits
     uint8_t* top_host = nullptr;     // pinned
     uint8_t *top_rows_dev = nullptr, *top_rows_host = nullptr;  // the same for every wanted row of a batch: [n_seq][TOP_BYTES]
+    void* top_scratch = nullptr;     // working memory of that reduction, for up to n_seq rows
     uint32_t* mask_dev = nullptr;    // allowed-token bits of a constrained pick
     float* ap_part = nullptr;        // partial results of the chunked prompt attention
     unsigned* ap_counters = nullptr;
@@ -416,7 +417,8 @@ int chunk(Model* m, const int32_t* tokens, int B, int pos0, float* logits, const
     if (top) {
         if (top->allowed)  // (pageable source: staged by the runtime before the call returns)
             ELB_CUDA(cudaMemcpyAsync(m->mask_dev, top->allowed, size_t((m->cfg.n_vocab + 31) / 32) * 4, cudaMemcpyHostToDevice, m->stream));
-        ELB_TRY(logits_top_launch(dev_logits, m->cfg.n_vocab, top->k, m->top_dev, m->stream, top->allowed ? m->mask_dev : nullptr));
+        ELB_TRY(logits_top_launch(dev_logits, m->cfg.n_vocab, 0, 1, top->k, m->top_dev, m->top_scratch, m->n_seq, m->stream,
+                                  top->allowed ? m->mask_dev : nullptr));
         ++m->launches;
     }
     ELB_CUDA(cudaEventRecord(m->ev1, m->stream));
@@ -733,7 +735,7 @@ void model_destroy(Model* m) {
     cudaFree(m->xr); cudaFree(m->logits_local);
     cudaFree(m->ap_part); cudaFree(m->ap_counters); cudaFree(m->top_dev); cudaFree(m->mask_dev);
     if (m->top_host) cudaFreeHost(m->top_host);
-    cudaFree(m->top_rows_dev);
+    cudaFree(m->top_rows_dev); cudaFree(m->top_scratch);
     if (m->top_rows_host) cudaFreeHost(m->top_rows_host);
     cudaFree(m->seq_dev); cudaFree(m->posv_dev); cudaFree(m->logits_rows); cudaFree(m->rows_part); cudaFree(m->rows_counters);
     tp_reduce_destroy(m->tpr);
@@ -932,6 +934,8 @@ static int finalize_local(Model* m) {
     ELB_CUDA(cudaMallocHost(&m->top_host, TOP_BYTES));
     ELB_CUDA(cudaMalloc(&m->top_rows_dev, size_t(m->n_seq) * TOP_BYTES));
     ELB_CUDA(cudaMallocHost(&m->top_rows_host, size_t(m->n_seq) * TOP_BYTES));
+    ELB_CUDA(cudaMalloc(&m->top_scratch, logits_top_scratch_bytes(int(V), m->n_seq)));
+    ELB_CUDA(cudaMemset(m->top_scratch, 0, logits_top_scratch_bytes(int(V), m->n_seq)));
     ELB_CUDA(cudaMalloc(&m->mask_dev, size_t((V + 31) / 32) * 4));
     ELB_CUDA(cudaMalloc(&m->ap_part, attn_prefill_scratch_floats(m->max_batch, m->H, m->HKV) * sizeof(float)));
     ELB_CUDA(cudaMalloc(&m->ap_counters, attn_prefill_counters(m->max_batch, m->H, m->HKV) * sizeof(unsigned)));
@@ -1107,7 +1111,7 @@ static int eval_batch_impl(Model* m, int n, const int32_t* tokens, const int32_t
         out_dev = m->logits_rows;
     }
     if (out_dev && top) {  // k best tokens and the log-sum-exp of every wanted row, on the device
-        ELB_TRY(logits_top_rows_launch(out_dev, int(V), V, int(rows.size()), top->k, m->top_rows_dev, m->stream));
+        ELB_TRY(logits_top_launch(out_dev, int(V), V, int(rows.size()), top->k, m->top_rows_dev, m->top_scratch, m->n_seq, m->stream));
         ++m->launches;
     }
     ELB_CUDA(cudaEventRecord(m->ev1, m->stream));
