@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "split.cuh"
+#include "attn_core.cuh"
 
 namespace elb {
 
@@ -530,9 +531,12 @@ __global__ void __launch_bounds__(AG_THREADS) k_attn_prefill_gqa(const float* __
 // ---------------------------------------------------------------- rows of several sequences
 
 // Row b of the batch is one token of sequence seqv[b] at position posv[b]; its q heads are normalised and rotated and
-// its K/V row is in the cache already (k_qkv_post). Grid (B, HKV, nsplit): all q heads of a KV group share one pass
-// over keys 0..posv[b] of that sequence; key splits meet in `part` and the last split to arrive adds them in split order.
-// The same arithmetic as k_attn_decode (src/model.cpp:191-214 of the reference).
+// its K/V row is in the cache already (k_qkv_post). Grid (B, HKV, most splits of a row): all q heads of a KV group share
+// one pass over keys 0..posv[b] of that sequence (attn_core.cuh), cut into ranges of about `per_split` keys so that rows
+// of different context lengths give CTAs of like work; the splits of a row meet in `part` and the last one to arrive
+// adds them in split order.
+// Bound by the K/V rows' bytes: 64 rows with 100-1000 keys on the 1.7B shape 111 -> 65 us per layer, 16 rows with 64-700
+// keys on the 4B shape 51 -> 27 us, against tiles staged in shared memory, scores by one warp per head and a CTA per row.
 struct AttnRowsParams {
     const float* qkv;
     int64_t ld;
@@ -543,162 +547,99 @@ struct AttnRowsParams {
     int64_t ld_att;
     float* part;         // [B][HKV][nsplit][group][D + 2]
     unsigned* counters;  // [B][HKV]
-    int H, HKV, nsplit;
+    int H, HKV, nsplit, per_split;
     float scale;
 };
 
-// Key / value tiles arrive by cp.async, the next tile while the current one is worked on: a CTA streams its whole key
-// range (a sequence's context when there are enough rows to fill the GPU without a key split), so the bytes in flight
-// per SM, not the arithmetic, set the pace.
-constexpr int AR_LDK = D + 4;  // key row stride: 16-byte aligned rows, conflict-free 128-bit reads (lane = key)
-constexpr int AR_KT = 24;       // keys per tile: two tiles of K and V are 50 KB, four CTAs per SM
-constexpr size_t AR_SMEM = size_t(2) * AR_KT * (AR_LDK + D) * sizeof(float);
+constexpr int AR_WARPS = 8, AR_THREADS = 32 * AR_WARPS;
 
-__global__ void __launch_bounds__(AD_THREADS) k_attn_rows(const AttnRowsParams p) {
-    extern __shared__ __align__(16) float ar_tiles[];
-    float* Ks = ar_tiles;                    // [2][AR_KT][AR_LDK]
-    float* Vs = Ks + 2 * AR_KT * AR_LDK;     // [2][AR_KT][D]
-    __shared__ __align__(16) float qs[AD_MAXG][D];
-    __shared__ float Ps[AD_MAXG][32];  // (a warp writes all 32 lanes)
-    __shared__ float corr_s[AD_MAXG], m_s[AD_MAXG], l_s[AD_MAXG];
+template <int GP>
+__global__ void __launch_bounds__(AR_THREADS, 2) k_attn_rows(const AttnRowsParams p) {
+    __shared__ __align__(16) float qs[GP * D];
+    __shared__ __align__(16) float work[ac_smem_floats(GP, AR_WARPS)];
     __shared__ int s_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int b = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, group = p.H / p.HKV, KD = p.HKV * D;
-    const int T = p.posv[b] + 1;
-    const float* kc = p.kc + size_t(p.seqv[b]) * p.seq_stride;
-    const float* vc = p.vc + size_t(p.seqv[b]) * p.seq_stride;
-    for (int idx = tid; idx < group * D; idx += AD_THREADS) qs[idx / D][idx % D] = p.qkv[int64_t(b) * p.ld + (kvh * group) * D + idx];
-    if (tid < AD_MAXG) { m_s[tid] = -INFINITY; l_s[tid] = 0.f; }
-    const int tiles = (T + AR_KT - 1) / AR_KT, per = (tiles + p.nsplit - 1) / p.nsplit;
-    const int t_begin = min(T, split * per * AR_KT), t_end = min(T, (split + 1) * per * AR_KT);
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};  // outputs (head tid/128 + 2i, dim tid%128)
-    const int od = tid & (D - 1), oh = tid >> 7;
-    auto fetch = [&](int buf, int t0, int nk) {
-        const unsigned ks = unsigned(__cvta_generic_to_shared(Ks + buf * AR_KT * AR_LDK));
-        const unsigned vs = unsigned(__cvta_generic_to_shared(Vs + buf * AR_KT * D));
-        for (int idx = tid; idx < nk * (D / 4); idx += AD_THREADS) {
-            const int j = idx / (D / 4), c = (idx % (D / 4)) * 4;
-            const size_t off = size_t(t0 + j) * KD + kvh * D + c;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ks + unsigned(j * AR_LDK + c) * 4u), "l"(kc + off));
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(vs + unsigned(j * D + c) * 4u), "l"(vc + off));
-        }
-        asm volatile("cp.async.commit_group;");
-    };
-    if (t_begin < t_end) fetch(0, t_begin, min(AR_KT, t_end - t_begin));
-    int buf = 0;
-    for (int t0 = t_begin; t0 < t_end; t0 += AR_KT, buf ^= 1) {
-        const int nk = min(AR_KT, t_end - t0);
-        if (t0 + AR_KT < t_end) {  // the other buffer was released by the barrier that ended the previous tile
-            fetch(buf ^ 1, t0 + AR_KT, min(AR_KT, t_end - t0 - AR_KT));
-            asm volatile("cp.async.wait_group 1;");
-        } else {
-            asm volatile("cp.async.wait_group 0;");
-        }
-        __syncthreads();
-        const float* Kb = Ks + buf * AR_KT * AR_LDK;
-        const float* Vb = Vs + buf * AR_KT * D;
-        if (warp < group) {  // scores: warp = head, lane = key; dimension order, multiply then add, as the CPU path does
-            float sc = -INFINITY;
-            if (lane < nk) {
-                float a = 0.f;
-                const float4* q = reinterpret_cast<const float4*>(qs[warp]);
-                const float4* kr = reinterpret_cast<const float4*>(Kb + lane * AR_LDK);
-#pragma unroll 8
-                for (int i = 0; i < D / 4; ++i) {
-                    const float4 qv = q[i], kv = kr[i];
-                    a = __fadd_rn(a, __fmul_rn(qv.x, kv.x));
-                    a = __fadd_rn(a, __fmul_rn(qv.y, kv.y));
-                    a = __fadd_rn(a, __fmul_rn(qv.z, kv.z));
-                    a = __fadd_rn(a, __fmul_rn(qv.w, kv.w));
-                }
-                sc = __fmul_rn(a, p.scale);
-            }
-            const float m_old = m_s[warp], m_new = fmaxf(m_old, warp_max(sc));
-            const float pj = lane < nk ? expf(sc - m_new) : 0.f;
-            const float sum = warp_sum(pj);
-            Ps[warp][lane] = pj;
-            if (lane == 0) {
-                const float c = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
-                corr_s[warp] = c;
-                l_s[warp] = l_s[warp] * c + sum;
-                m_s[warp] = m_new;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int h = oh + 2 * i;
-            if (h >= group) continue;
-            float a = acc[i] * corr_s[h];
-            if (nk == AR_KT) {  // a whole tile: fixed trip count, the loads run ahead of the additions
-#pragma unroll
-                for (int j = 0; j < AR_KT; ++j) a = fmaf(Ps[h][j], Vb[j * D + od], a);
-            } else {
-                for (int j = 0; j < nk; ++j) a = fmaf(Ps[h][j], Vb[j * D + od], a);
-            }
-            acc[i] = a;
-        }
-        __syncthreads();  // the tile and Ps are free again
-    }
-    __syncthreads();
-    float* out = p.att + int64_t(b) * p.ld_att;
-    if (p.nsplit == 1) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int h = oh + 2 * i;
-            if (h < group) out[(kvh * group + h) * D + od] = acc[i] / l_s[h];
-        }
-        return;
-    }
+    const int T = p.posv[b] + 1, ns = min(p.nsplit, (T + p.per_split - 1) / p.per_split);
+    if (split >= ns) return;
+    const float* kc = p.kc + size_t(p.seqv[b]) * p.seq_stride + kvh * D;
+    const float* vc = p.vc + size_t(p.seqv[b]) * p.seq_stride + kvh * D;
+    for (int idx = tid; idx < GP * D; idx += AR_THREADS) qs[idx] = idx < group * D ? p.qkv[int64_t(b) * p.ld + (kvh * group) * D + idx] : 0.f;
+    const AcSmem s = ac_smem(work, qs, GP, AR_WARPS);
+    const int t0 = int(int64_t(T) * split / ns), t1 = int(int64_t(T) * (split + 1) / ns);
+    float* out = p.att + int64_t(b) * p.ld_att + kvh * group * D;
     float* base = p.part + (size_t(b) * p.HKV + kvh) * p.nsplit * group * (D + 2);
     float* mine = base + size_t(split) * group * (D + 2);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int h = oh + 2 * i;
-        if (h < group) mine[h * (D + 2) + od] = acc[i];
-    }
+    constexpr int KT = 32 / GP < 8 ? 32 / GP : 8;
+    AcKeys<GP, KT, AR_WARPS> keys(kc, vc, size_t(KD), t0, t1, warp, lane);
+    keys.first(-1);
+    __syncthreads();
+    keys.walk(-1, nullptr, nullptr, s, p.scale);
+    ac_finish<GP, KT, AR_WARPS>(keys.w, s, group, warp, lane, [] { __syncthreads(); }, [&](int h, int d, float o) {
+        if (ns == 1) out[h * D + d] = o / s.l[h];
+        else mine[h * (D + 2) + d] = o;
+    });
+    if (ns == 1) return;
     if (tid < group) {
-        mine[tid * (D + 2) + D] = m_s[tid];
-        mine[tid * (D + 2) + D + 1] = l_s[tid];
+        mine[tid * (D + 2) + D] = s.m[tid];
+        mine[tid * (D + 2) + D + 1] = s.l[tid];
     }
     __threadfence();
     __syncthreads();
     if (tid == 0) {
         unsigned* cnt = p.counters + size_t(b) * p.HKV + kvh;
         const unsigned old = atomicAdd(cnt, 1u);
-        s_last = old == unsigned(p.nsplit - 1);
+        s_last = old == unsigned(ns - 1);
         if (s_last) *cnt = 0;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int h = oh + 2 * i;
-        if (h >= group) continue;
+    for (int e = tid; e < group * D; e += AR_THREADS) {
+        const int h = e / D, od = e % D;
         float M = -INFINITY;
-        for (int q = 0; q < p.nsplit; ++q) M = fmaxf(M, __ldcg(base + (size_t(q) * group + h) * (D + 2) + D));
+        for (int q = 0; q < ns; ++q) M = fmaxf(M, __ldcg(base + (size_t(q) * group + h) * (D + 2) + D));
         float L = 0.f, o = 0.f;
-        for (int q = 0; q < p.nsplit; ++q) {  // fixed split order
+#pragma unroll 4
+        for (int q = 0; q < ns; ++q) {  // fixed split order
             const float* ps = base + (size_t(q) * group + h) * (D + 2);
-            const float mq = __ldcg(ps + D);
-            if (mq == -INFINITY) continue;
-            const float w = expf(mq - M);
+            const float w = expf(__ldcg(ps + D) - M);
             L = fmaf(__ldcg(ps + D + 1), w, L);
             o = fmaf(__ldcg(ps + od), w, o);
         }
-        out[(kvh * group + h) * D + od] = o / L;
+        out[e] = o / L;
     }
 }
 
+// Most splits a row can have when the batch has B rows: the partial results of AR_ROW_SPLITS (row, split) pairs fit.
+constexpr int AR_ROW_SPLITS = 2048, AR_MAXSPLIT = 32;
+static int attn_rows_most_splits(int B) { return std::max(1, std::min(AR_MAXSPLIT, AR_ROW_SPLITS / std::max(B, 1))); }
+size_t attn_rows_part_floats(int H) { return size_t(AR_ROW_SPLITS) * H * (D + 2); }
+
+// posv_host: the rows' positions on the host (they decide how the keys are cut)
 int attn_rows_launch(const float* qkv, int64_t ld, const float* kc, const float* vc, size_t seq_stride, const int* posv,
-                     const int* seqv, float* att, int64_t ld_att, float* part, unsigned* counters, int B, int H, int HKV,
-                     int nsplit, float scale, cudaStream_t s) {
+                     const int* seqv, const int* posv_host, float* att, int64_t ld_att, float* part, unsigned* counters, int B, int H,
+                     int HKV, float scale, int sm_count, cudaStream_t s) {
     if (H % HKV || H / HKV > AD_MAXG) return fail(ELB_ERR_UNSUPPORTED, "attention: at most 8 query heads per KV head");
-    if (nsplit < 1 || nsplit > AD_MAXSPLIT) return fail(ELB_ERR_INVALID, "attention: split count out of range");
-    AttnRowsParams p{qkv, ld, kc, vc, seq_stride, posv, seqv, att, ld_att, part, counters, H, HKV, nsplit, scale};
-    ELB_TRY(ensure_dyn_smem((const void*)k_attn_rows, AR_SMEM));
-    k_attn_rows<<<dim3(B, HKV, nsplit), AD_THREADS, AR_SMEM, s>>>(p);
+    // Ranges of 256 keys, halved (down to 64: below that the fixed cost of a CTA and of the combination outweighs its keys)
+    // until the GPU has two CTAs per SM.
+    int Tmax = 1;
+    for (int b = 0; b < B; ++b) Tmax = std::max(Tmax, posv_host[b] + 1);
+    int per = 256;
+    for (; per > 64; per /= 2) {
+        int64_t ctas = 0;
+        for (int b = 0; b < B; ++b) ctas += (posv_host[b] + per) / per;
+        if (ctas * HKV >= 2 * int64_t(sm_count)) break;
+    }
+    const int most = attn_rows_most_splits(B);
+    if ((Tmax + per - 1) / per > most) per = (Tmax + most - 1) / most;
+    const int nsplit = (Tmax + per - 1) / per;
+    AttnRowsParams p{qkv, ld, kc, vc, seq_stride, posv, seqv, att, ld_att, part, counters, H, HKV, nsplit, per, scale};
+    const dim3 grid{unsigned(B), unsigned(HKV), unsigned(nsplit)};
+    const int group = H / HKV;
+    if (group <= 2) k_attn_rows<2><<<grid, AR_THREADS, 0, s>>>(p);
+    else if (group <= 4) k_attn_rows<4><<<grid, AR_THREADS, 0, s>>>(p);
+    else k_attn_rows<8><<<grid, AR_THREADS, 0, s>>>(p);
     ELB_CUDA(cudaGetLastError());
     return ELB_OK;
 }

@@ -270,10 +270,12 @@ int attn_decode_launch(const AttnDecodeArgs& a, cudaStream_t s);
 int qkv_post_launch(float* qkv, int64_t ld, const float* q_norm, const float* k_norm, const float* rope, int pos0, int B,
                     float* kc, float* vc, int H, int HKV, int rope_dim, float eps, cudaStream_t s,
                     const int* posv = nullptr, const int* seqv = nullptr, size_t seq_stride = 0);
-// rows of several sequences (row b: position posv[b] of sequence seqv[b]); part [B][HKV][nsplit][group][130], counters [B][HKV]
+// rows of several sequences (row b: position posv[b] of sequence seqv[b]; posv_host: the positions on the host); part:
+// attn_rows_part_floats(H) floats, counters [B][HKV] zero at first
+size_t attn_rows_part_floats(int H);
 int attn_rows_launch(const float* qkv, int64_t ld, const float* kc, const float* vc, size_t seq_stride, const int* posv,
-                     const int* seqv, float* att, int64_t ld_att, float* part, unsigned* counters, int B, int H, int HKV,
-                     int nsplit, float scale, cudaStream_t s);
+                     const int* seqv, const int* posv_host, float* att, int64_t ld_att, float* part, unsigned* counters, int B, int H,
+                     int HKV, float scale, int sm_count, cudaStream_t s);
 int attn_prefill_launch(const float* qkv, int64_t ld, const float* kc, const float* vc, float* att, int64_t ld_att,
                         int pos0, int B, int H, int HKV, float scale, cudaStream_t s, float* part = nullptr,
                         unsigned* counters = nullptr);

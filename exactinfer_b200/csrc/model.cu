@@ -41,7 +41,7 @@ bool env_on(const char* name) {
 
 struct Model {
     elb_config cfg{};
-    int n_ctx = 0, device = 0, max_batch = 512, n_seq = 1;
+    int n_ctx = 0, device = 0, max_batch = 512, n_seq = 1, sm_count = 0;
     bool finalized = false;
     std::vector<HostTensor> pending;  // [3 + n_layer * 11], valid until finalize
     cudaStream_t stream = nullptr;
@@ -99,7 +99,6 @@ struct Model {
     float* logits_rows = nullptr;                  // [n_seq][n_vocab] logits of the wanted rows of a batch
     float* rows_part = nullptr;                    // attention partial results of a batch
     unsigned* rows_counters = nullptr;
-    int rows_split = 1;
     uint8_t* top_dev = nullptr;      // device-side logits post-processing: lse, ids, logits
     uint8_t* top_host = nullptr;     // pinned
     uint8_t *top_rows_dev = nullptr, *top_rows_host = nullptr;  // the same for every wanted row of a batch: [n_seq][TOP_BYTES]
@@ -217,7 +216,9 @@ int rows_all_reduce(Model* m, int B) {
 }
 
 // Rows of one sequence at consecutive positions (seq0, pos0 + b), or (mixed) row b at posv_dev[b] of sequence seq_dev[b].
-int body_prefill(Model* m, int B, int pos0, int seq0 = 0, bool mixed = false) {
+// posv_host (mixed): the positions on the host.
+int body_prefill(Model* m, int B, int pos0, int seq0 = 0, const int* posv_host = nullptr) {
+    const bool mixed = posv_host != nullptr;
     const elb_config& c = m->cfg;
     const int E = c.n_embd, F = int(m->F), H = m->H, HKV = m->HKV, QD = H * 128, KD = HKV * 128, QKV = QD + 2 * KD;
     const float scale = 1.0f / std::sqrt(float(c.head_dim));
@@ -239,8 +240,8 @@ int body_prefill(Model* m, int B, int pos0, int seq0 = 0, bool mixed = false) {
         if (mixed) {
             ELB_TRY(qkv_post_launch(m->qkv, QKV, L.q_norm, L.k_norm, m->rope, 0, B, kc, vc, H, HKV, c.rope_dim, c.eps, m->stream,
                                     m->posv_dev, m->seq_dev, seq_stride));
-            ELB_TRY(attn_rows_launch(m->qkv, QKV, kc, vc, seq_stride, m->posv_dev, m->seq_dev, m->att, QD, m->rows_part,
-                                     m->rows_counters, B, H, HKV, m->rows_split, scale, m->stream));
+            ELB_TRY(attn_rows_launch(m->qkv, QKV, kc, vc, seq_stride, m->posv_dev, m->seq_dev, posv_host, m->att, QD,
+                                     m->rows_part, m->rows_counters, B, H, HKV, scale, m->sm_count, m->stream));
         } else {
             ELB_TRY(qkv_post_launch(m->qkv, QKV, L.q_norm, L.k_norm, m->rope, pos0, B, kc, vc, H, HKV, c.rope_dim, c.eps, m->stream));
             if (m->kv16 && attn_prefill_tc_usable(H, HKV, QKV, QD)) {
@@ -900,15 +901,10 @@ static int finalize_local(Model* m) {
     ELB_CUDA(cudaMalloc(&m->tokens_dev, size_t(B) * sizeof(int32_t)));
     ELB_CUDA(cudaMalloc(&m->pos_dev, sizeof(int)));
     if (m->n_seq > 1) {
-        DeviceInfo dinfo;
-        ELB_TRY(device_info(m->device, &dinfo));
         ELB_CUDA(cudaMalloc(&m->seq_dev, size_t(B) * sizeof(int)));
         ELB_CUDA(cudaMalloc(&m->posv_dev, size_t(B) * sizeof(int)));
         ELB_CUDA(cudaMalloc(&m->logits_rows, size_t(m->n_seq) * V * sizeof(float)));
-        // key splits of the batched attention: enough CTAs for two per SM when one row per sequence is in the batch
-        m->rows_split = int(std::max<int64_t>(1, std::min<int64_t>(8, (2 * dinfo.sm_count + int64_t(m->n_seq) * m->HKV - 1) / (int64_t(m->n_seq) * m->HKV))));
-        const int group = c.n_head / c.n_head_kv;
-        ELB_CUDA(cudaMalloc(&m->rows_part, size_t(B) * m->HKV * m->rows_split * group * (128 + 2) * sizeof(float)));
+        ELB_CUDA(cudaMalloc(&m->rows_part, attn_rows_part_floats(m->H) * sizeof(float)));
         ELB_CUDA(cudaMalloc(&m->rows_counters, size_t(B) * m->HKV * sizeof(unsigned)));
         ELB_CUDA(cudaMemset(m->rows_counters, 0, size_t(B) * m->HKV * sizeof(unsigned)));
     }
@@ -924,6 +920,7 @@ static int finalize_local(Model* m) {
     // decode attention: a fixed number of key splits so that the launch shape does not depend on the position
     DeviceInfo di;
     ELB_TRY(device_info(m->device, &di));
+    m->sm_count = di.sm_count;
     m->attn_split = std::max(1, std::min(32, (di.sm_count + m->HKV - 1) / m->HKV));
     if (const char* v = std::getenv("ELB_ATTN_SPLIT")) m->attn_split = std::max(1, std::min(32, std::atoi(v)));
     const int group = c.n_head / c.n_head_kv;
@@ -1083,7 +1080,7 @@ static int eval_batch_impl(Model* m, int n, const int32_t* tokens, const int32_t
     ELB_CUDA(cudaEventRecord(m->ev0, m->stream));
     ELB_TRY(launch_gather_rows(m->embd, m->tokens_dev, n, m->x, m->stream));
     ++m->launches;
-    ELB_TRY(body_prefill(m, n, pos[0], seq[0], !uniform));
+    ELB_TRY(body_prefill(m, n, pos[0], seq[0], uniform ? nullptr : pos));
     m->last_rows = n;
     float* out_dev = nullptr;
     if (rows.size() == 1) {
