@@ -12,6 +12,9 @@ constexpr int DK_MAX_LAYERS = 96;  // layers a model may have to run on this ker
 constexpr int DK_KINDS = 7;        // 0..2 qkv segment, 3 attn_output, 4 gate|up, 5 ffn_down, 6 head
 constexpr int DK_LAYER_MATS = 6;   // matrices of a layer in execution order: n_qkv segments, attn_output, gate|up, ffn_down
 
+constexpr int DK_MAX_PARTS = 4;     // most parts ffn_down is cut into along k (decode_one.cu)
+constexpr int DK_ONE_KINDS = 6 + DK_MAX_PARTS;
+
 struct DkKind {  // one kind of weight matrix, in tiled layout
     int tiles, upt, rows, n;
     // How the CTAs share the matrix. group_tiles / group_off: the matrix is tiles [group_off, group_off + tiles) of a
@@ -40,6 +43,7 @@ struct DkParams {
     int embd_type;
     int E, F, H, HKV, rope_dim, n_ctx, nsplit;
     float eps, scale;
+    double inv_E;           // 1 / E
     int nl_qkv, nl_wo, nl_gu, nl_down;
     const int32_t* token;   // device arrays: token id and position of step i of the running batch of steps
     const int* pos;
@@ -71,11 +75,32 @@ struct DkParams {
     int slots;              // row-tile slots per warp in the reduction buffer
     int cta_tiles;          // most row tiles a CTA's share of a matrix can touch
     int n_max;              // longest activation vector
+    // decode_one.cu: the vectors that pass between CTAs, each twice (one half per layer, in turn)
+    float *ex_e, *ex_q, *ex_a, *ex_p1, *ex_g, *ex_p2, *ex_s;  // embedding row, q|k|v, att, partial sums [2][E], act, partial sums, attention splits
+    unsigned* fin;          // CTAs that have finished the step (zero between launches)
+    int qkv_len;            // floats of q|k|v
+    const uint8_t* f16_maps;  // F16: tensor maps of the matrices [n_layer + 1][DK_LAYER_MATS]
+    int f16;                // every matrix is F16 (otherwise every one is quantized)
+    int down_parts;         // equal ranges of k in which ffn_down is worked off
+    int down_blocks;        // 256-value blocks of the activation in one of them
+    // by kind of matrix (0..2 q|k|v, attn_output, gate|up, head, the parts of ffn_down): units of a row tile, first row-tile
+    // slot in the reduction buffer (kinds of one stage side by side), first entry in the table of a CTA's row tiles
+    int upt1[DK_ONE_KINDS], slot_base[DK_ONE_KINDS], tile_base[DK_ONE_KINDS + 1];
     unsigned long long* prof;  // diagnostics (ELB_DK_PROF=1): [n_layer][32] nanosecond stamps of CTA 0, else null
     unsigned long long* prof_cta;  // diagnostics: [CTAs][16] stamps of every CTA at the barriers of layer prof_layer (arrival, release)
     int prof_layer;
 };
 
+// decode_one.cu (one GPU)
+size_t decode_one_exchange(DkParams& p, float* base);
+int decode_one_ring_bytes(const DkParams& p, int max_unit, int min_unit, int device);
+int decode_one_fits(const DkParams& p, int ring_bytes, int device, bool* fits);
+int decode_one_launch(const DkParams& p, int ring_bytes, int grid, cudaStream_t s);
+int decode_one_f16_unit();
+bool decode_one_f16_maps(const DkParams& p, void* host);
+int decode_one_warps();
+
+// decode.cu (tensor parallelism, and shapes that decode_one.cu does not take)
 // one token at the position / token id stored on the device (step ctl[0] of the arrays); nothing to reset between launches.
 // ring_bytes: size of one warp's ring of weight units in shared memory (decode_ring_bytes); grid: one CTA per SM.
 int decode_step_launch(const DkParams& p, int ring_bytes, int grid, cudaStream_t s);

@@ -82,6 +82,9 @@ struct Model {
     float* xbuf = nullptr;  // persistent kernel: residual stream [2][E]
     TpPeerBuf xarea;        // persistent kernel: flags, partial sums and logits, visible to all tensor-parallel ranks
     unsigned* xctl = nullptr;
+    bool one = false;            // single GPU: decode_one.cu
+    float* exchange = nullptr;   // its exchange buffers
+    uint8_t* f16_maps = nullptr; // its tensor maps (F16 models)
     int8_t* gact = nullptr;  // persistent kernel: limbs of the FFN activation when they do not fit in shared memory
     float* logits_step = nullptr;  // where a single-token step leaves its logits (m->logits unless the persistent kernel runs)
     unsigned* sync_words = nullptr;  // barrier counter, step index, advance flag, launch count, then 2 x [n_layer][2] amax slots
@@ -338,7 +341,7 @@ int body_decode(Model* m) {
     };
     if (m->use_mega) {
         ++m->launches;
-        return decode_step_launch(m->dk, m->dk_slot, m->dk_grid, m->stream);
+        return m->one ? decode_one_launch(m->dk, m->dk_slot, m->dk_grid, m->stream) : decode_step_launch(m->dk, m->dk_slot, m->dk_grid, m->stream);
     }
     auto quant = [](const Weight* w) { return w->type != ELB_F16; };
     auto qkv_quant = [&](const Layer& L) { bool q = false; for (auto& s : L.qkv) q |= quant(s.w); return q; };
@@ -445,6 +448,172 @@ int chunk(Model* m, const int32_t* tokens, int B, int pos0, float* logits, const
 }
 
 }  // namespace
+
+// The persistent decode kernel for one GPU (decode_one.cu): every matrix quantized, or every matrix F16. Leaves m->one
+// false when the model's shape is not one of its shapes.
+static int setup_decode_one(Model* m) {
+    const elb_config& c = m->cfg;
+    if (m->tp.size > 1 || env_on("ELB_NO_MEGA") || env_on("ELB_DK_OLD")) return ELB_OK;
+    DeviceInfo di;
+    ELB_TRY(device_info(m->device, &di));
+    const int E = c.n_embd, F = int(m->F), QD = m->H * 128, KD = m->HKV * 128, L = c.n_layer, group = m->H / m->HKV;
+    const size_t nq = m->layers[0].qkv.size();
+    const bool f16 = m->head->type == ELB_F16;
+    if (m->embd->type == ELB_F32 || nq > 3 || E % 256 || F % 256 || QD % 256 || L > DK_MAX_LAYERS || E / 256 > di.sm_count) return ELB_OK;
+    auto upt = [&](const Weight* w) { return f16 ? int(w->n / 128) : int(w->units_per_tile); };
+    auto like = [](const Weight* a, const Weight* b) { return a->rows == b->rows && a->n == b->n; };
+    for (const Layer& y : m->layers) {  // the shapes of layer 0 in every layer; block formats may differ
+        const Layer& y0 = m->layers[0];
+        bool ok = y.qkv.size() == nq && like(y.wo, y0.wo) && like(y.gu, y0.gu) && like(y.down, y0.down);
+        for (size_t i = 0; ok && i < nq; ++i) ok = like(y.qkv[i].w, y0.qkv[i].w) && y.qkv[i].col == y0.qkv[i].col && (y.qkv[i].w->type == ELB_F16) == f16;
+        ok = ok && (y.wo->type == ELB_F16) == f16 && (y.gu->type == ELB_F16) == f16 && (y.down->type == ELB_F16) == f16;
+        // (a unit is 256 values of k for some formats and 128 for others: the kernel knows one number per kind of matrix)
+        for (size_t i = 0; ok && i < nq; ++i) ok = upt(y.qkv[i].w) == upt(y0.qkv[i].w);
+        if (!ok || upt(y.wo) != upt(y0.wo) || upt(y.gu) != upt(y0.gu) || upt(y.down) != upt(y0.down)) return ELB_OK;
+    }
+    DkParams& p = m->dk;
+    p = DkParams{};
+    p.f16 = f16;
+    auto kind_of = [&](const Weight* w) { return DkKind{int(w->tiles), upt(w), int(w->rows), int(w->n), int(w->tiles), 0, 0, 0}; };
+    // equal unit ranges when every CTA's range is at least one tile long: a tile then has at most two contributors
+    auto kind_balanced = [&](const Weight* w) {
+        DkKind d = kind_of(w);
+        d.balanced = w->tiles >= di.sm_count ? 1 : 0;
+        return d;
+    };
+    int unit_max = 0, unit_min = 1 << 30;
+    auto account = [&](const Weight* w) {
+        const int ub = f16 ? decode_one_f16_unit() : w->unit_bytes;
+        unit_max = std::max(unit_max, ub);
+        unit_min = std::min(unit_min, ub);
+    };
+    const Layer& L0 = m->layers[0];
+    int group_tiles = 0;
+    for (size_t i = 0; i < nq; ++i) group_tiles += int(L0.qkv[i].w->tiles);
+    for (size_t i = 0, off = 0; i < nq; ++i) {  // q, k, v share one phase: the CTAs cut the tiles of all three together
+        p.kind[i] = kind_of(L0.qkv[i].w);
+        p.kind[i].group_tiles = group_tiles;
+        p.kind[i].group_off = int(off);
+        p.qkv_col[i] = int(L0.qkv[i].col);
+        off += size_t(L0.qkv[i].w->tiles);
+    }
+    p.kind[3] = kind_balanced(L0.wo); p.kind[4] = kind_of(L0.gu); p.kind[5] = kind_balanced(L0.down); p.kind[6] = kind_of(m->head);
+    for (int l = 0; l < L; ++l) {
+        const Layer& y = m->layers[size_t(l)];
+        const Weight* mats[6];
+        size_t n = 0;
+        for (auto& s : y.qkv) mats[n++] = s.w;
+        for (const Weight* w : {y.wo, y.gu, y.down}) mats[n++] = w;
+        for (size_t i = 0; i < n; ++i) {
+            p.W[l][i] = mats[i]->tiled;
+            p.wtype[l][i] = uint8_t(mats[i]->type);
+            account(mats[i]);
+        }
+    }
+    p.W[L][0] = m->head->tiled;
+    p.wtype[L][0] = uint8_t(m->head->type);
+    account(m->head);
+    if (nq > 1) {  // q|k|v cut by cost: a tile's units times the time a unit of its format takes
+        auto unit_cost = [](int type) { return type == ELB_Q6_K ? 1455 : type == ELB_Q8_0 ? 481 : 875; };  // SM clocks, measured
+        long long off = 0;
+        for (size_t i = 0; i < nq; ++i) {
+            long long sum = 0;
+            for (int l = 0; l < L; ++l) sum += unit_cost(p.wtype[l][i]);
+            p.kind[i].cost = int(sum / L) * p.kind[i].upt;
+            p.kind[i].group_cost_off = int(off);
+            off += (long long)p.kind[i].cost * p.kind[i].tiles;
+        }
+        if (off < (1ll << 30))
+            for (size_t i = 0; i < nq; ++i) p.kind[i].group_cost = int(off);
+    }
+    for (int i = 0; i < 7; ++i)  // 32-bit unit arithmetic in the kernel
+        if (int64_t(p.kind[i].tiles) * p.kind[i].upt * di.sm_count >= (int64_t(1) << 31)) return ELB_OK;
+    p.n_layer = L; p.n_qkv = int(nq);
+    p.norms = m->norm_arena;
+    p.norm_stride = int(2 * E + 2 * c.head_dim);
+    p.kc = m->kcache; p.vc = m->vcache;  // sequence 0
+    p.kv_stride = size_t(m->n_seq) * m->n_ctx * KD;
+    p.output_norm = m->output_norm;
+    p.embd = m->embd->tiled; p.embd_type = m->embd->type;
+    p.E = E; p.F = F; p.H = m->H; p.HKV = m->HKV; p.rope_dim = c.rope_dim; p.n_ctx = m->n_ctx;
+    p.qkv_len = QD + 2 * KD;
+    p.nsplit = std::max(1, std::min(decode_max_split(), di.sm_count / m->HKV));
+    p.tp_size = 1;
+    p.eps = c.eps; p.scale = 1.0f / std::sqrt(float(c.head_dim)); p.inv_E = 1.0 / E;
+    p.nl_qkv = m->nl_qkv; p.nl_wo = m->nl_wo; p.nl_gu = m->nl_gu; p.nl_down = m->nl_down;
+    p.rope = m->rope; p.x = m->x;
+    p.logits_peer[0] = m->logits;
+    if (m->HKV > di.sm_count || group > 8) return ELB_OK;
+    // Rings and activation share an SM's memory: ffn_down's activation is worked off in as many equal parts as leave the
+    // rings 8 KB per warp (three to four units of weights).
+    const int min_ring = std::max(8192, 2 * unit_max);
+    bool fits = false;
+    for (p.down_parts = 1; p.down_parts <= DK_MAX_PARTS && !fits; ++p.down_parts) {
+        if (p.kind[5].upt % p.down_parts || (F / 256) % p.down_parts) continue;
+        p.n_max = std::max({E, QD, F / p.down_parts});
+        // row-tile slots of the reduction buffer: what one warp's share of each kind can touch; kinds of a stage side by side
+        auto slots_of = [&](const DkKind& k, int u) {
+            const int64_t per_cta = (int64_t(k.tiles) + di.sm_count - 1) / di.sm_count * u, per_warp = (per_cta + decode_one_warps() - 1) / decode_one_warps();
+            return int((per_warp + u - 1) / u + 2);
+        };
+        int used = 0, most = 0, tiles = 0;
+        for (size_t i = 0; i < nq; ++i) {
+            p.slot_base[i] = used;
+            // (by cost a CTA can have more tiles of a cheap format than its share by count)
+            used += 2 * slots_of(p.kind[i], p.kind[i].upt);
+        }
+        most = used;
+        p.slot_base[3] = p.slot_base[4] = p.slot_base[5] = 0;
+        most = std::max({most, slots_of(p.kind[3], p.kind[3].upt), slots_of(p.kind[4], p.kind[4].upt), slots_of(p.kind[6], p.kind[6].upt)});
+        used = 0;
+        for (int h = 0; h < p.down_parts; ++h) { p.slot_base[6 + h] = used; used += slots_of(p.kind[5], p.kind[5].upt / p.down_parts); }
+        p.slots = std::max(most, used);
+        p.down_blocks = F / 256 / p.down_parts;
+        for (int i = 0, at = 0; i < DK_ONE_KINDS; ++i) {
+            const DkKind& k = p.kind[i < 5 ? i : i == 5 ? 6 : 5];
+            p.upt1[i] = i < 6 ? k.upt : k.upt / p.down_parts;
+            p.tile_base[i] = at;
+            at += ((k.tiles + di.sm_count - 1) / di.sm_count + 2) * (i < 3 ? 3 : 1);
+            p.tile_base[i + 1] = at;
+        }
+        for (int i : {3, 5}) tiles = std::max(tiles, (p.kind[i].tiles + di.sm_count - 1) / di.sm_count + 2);
+        p.cta_tiles = tiles;  // of the row-parallel matrices: rows of the residual stream a CTA keeps
+        m->dk_slot = decode_one_ring_bytes(p, unit_max, unit_min, m->device);
+        if (m->dk_slot < min_ring) continue;
+        ELB_TRY(decode_one_fits(p, m->dk_slot, m->device, &fits));
+        if (fits) break;
+    }
+    int coop = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device) != cudaSuccess) { cudaGetLastError(); coop = 0; }
+    if (!fits || !coop) return ELB_OK;
+    if (f16) {
+        std::vector<uint8_t> maps(size_t(L + 1) * DK_LAYER_MATS * 128);
+        if (!decode_one_f16_maps(p, maps.data())) return ELB_OK;
+        ELB_CUDA(cudaMalloc(&m->f16_maps, maps.size()));
+        ELB_CUDA(cudaMemcpy(m->f16_maps, maps.data(), maps.size(), cudaMemcpyHostToDevice));
+        p.f16_maps = m->f16_maps;
+    }
+    const size_t xfloats = decode_one_exchange(p, nullptr);
+    ELB_CUDA(cudaMalloc(&m->exchange, xfloats * sizeof(float)));
+    ELB_CUDA(cudaMemset(m->exchange, 0xFF, xfloats * sizeof(float)));  // every word empty
+    decode_one_exchange(p, m->exchange);
+    ELB_CUDA(cudaMalloc(&m->sync_words, 4 * sizeof(unsigned)));
+    ELB_CUDA(cudaMemset(m->sync_words, 0, 4 * sizeof(unsigned)));
+    ELB_CUDA(cudaMalloc(&m->pos_steps, size_t(m->max_batch) * sizeof(int)));
+    ELB_CUDA(cudaHostAlloc(&m->err_host, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+    *m->err_host = 0;
+    ELB_CUDA(cudaHostGetDevicePointer(&p.err, m->err_host, 0));
+    p.token = m->tokens_dev; p.pos = m->pos_steps;
+    p.fin = m->sync_words; p.ctl = m->sync_words + 1;
+    m->dk_grid = di.sm_count;
+    m->use_mega = m->one = true;
+    m->logits_step = m->logits;
+    if (env_on("ELB_DK_PROF")) {
+        ELB_CUDA(cudaMalloc(&p.prof, size_t(L + 1) * 32 * sizeof(unsigned long long)));
+        ELB_CUDA(cudaMemset(p.prof, 0, size_t(L + 1) * 32 * sizeof(unsigned long long)));
+    }
+    return ELB_OK;
+}
 
 // Fill the parameters of the persistent decode kernel; it is used when every weight is quantized and the step's
 // shared memory (rings + the longest activation's limbs) fits on one SM. ELB_NO_MEGA=1 keeps the kernel-per-op path.
@@ -731,7 +900,7 @@ void model_destroy(Model* m) {
                     (void*)m->tokens_dev, (void*)m->pos_dev, (void*)m->attn_part, (void*)m->attn_counters, (void*)m->dlimbs[0],
                     (void*)m->dlimbs[1], (void*)m->dlimbs[2], (void*)m->dlimbs[3], (void*)m->dinv, (void*)m->done})
         cudaFree(p);
-    cudaFree(m->xbuf); cudaFree(m->xctl); cudaFree(m->gact); cudaFree(m->tc_part); cudaFree(m->tc_counters); cudaFree(m->kv16);
+    cudaFree(m->exchange); cudaFree(m->f16_maps); cudaFree(m->xbuf); cudaFree(m->xctl); cudaFree(m->gact); cudaFree(m->tc_part); cudaFree(m->tc_counters); cudaFree(m->kv16);
     if (m->xarea.local) tp_peer_free(&m->xarea, m->tp.rank); cudaFree(m->sync_words); cudaFree(m->pos_steps);
     cudaFree(m->xr); cudaFree(m->logits_local);
     cudaFree(m->ap_part); cudaFree(m->ap_counters); cudaFree(m->top_dev); cudaFree(m->mask_dev);
@@ -970,7 +1139,8 @@ int model_finalize(Model* m) {
     } else if (rc != ELB_OK) {
         return rc;
     }
-    const int rc_k = setup_decode_kernel(m, rc == ELB_OK);
+    int rc_k = rc == ELB_OK ? setup_decode_one(m) : ELB_OK;
+    if (!m->one && rc_k == ELB_OK) rc_k = setup_decode_kernel(m, rc == ELB_OK);
     if (rc == ELB_OK) rc = rc_k;
     if (tp) {
         bool all = false;
@@ -1178,6 +1348,26 @@ int model_eval_steps(Model* m, const int32_t* tokens, int n, int pos0, float* de
     if (m->use_mega && m->dk.prof) {  // diagnostics: phase times of the last step, CTA 0, averaged over the layers
         std::vector<unsigned long long> t(size_t(m->cfg.n_layer) * 32);
         cudaMemcpy(t.data(), m->dk.prof, t.size() * 8, cudaMemcpyDeviceToHost);
+        if (m->one) {
+            static const char* n1[12] = {"", "convert qkv", "matvec qkv", "attention", "convert wo", "matvec wo", "", "convert gu", "matvec gu", "", "convert down", "matvec down"};
+            double total = 0;
+            for (int ev = 1, before = 0; ev < 12; ++ev) {
+                if (!n1[ev][0]) continue;
+                double sum = 0;
+                for (int l = 0; l < m->cfg.n_layer; ++l) sum += double(t[size_t(l) * 32 + ev] - t[size_t(l) * 32 + before]);
+                std::fprintf(stderr, "[dk prof] %-13s %7.2f us\n", n1[ev], sum / m->cfg.n_layer / 1000.0);
+                total += sum / m->cfg.n_layer / 1000.0;
+                before = ev;
+            }
+            for (int ev = 12, before = 2; ev < 14; before = ev++) {
+                double sum = 0;
+                for (int l = 0; l < m->cfg.n_layer; ++l) sum += double(t[size_t(l) * 32 + ev] - t[size_t(l) * 32 + before]);
+                std::fprintf(stderr, "[dk prof] (%s %7.2f us)\n", ev == 12 ? "heads" : "keys ", sum / m->cfg.n_layer / 1000.0);
+            }
+            std::fprintf(stderr, "[dk prof] layer total   %7.2f us\n", total);
+            m->last_rows = 1;
+            return ELB_OK;
+        }
         static const char* names[15] = {"", "convert qkv", "matvec qkv", "barrier", "attention", "barrier", "convert wo", "matvec wo", "barrier", "convert gu", "matvec gu", "barrier", "convert down", "matvec down", "barrier"};
         double layer_total = 0;
         for (int ev = 1; ev < 15; ++ev) {

@@ -72,3 +72,41 @@ def test_top_tokens_at_chunk_edges(elb, vocab):
             assert np.array_equal(ids[r], order) and np.array_equal(vals[r], full[r][order])
             assert abs(lse[r] - ol.logsumexp(full[r])) <= 1e-12 * max(1.0, abs(lse[r]))
     gpu.close()
+
+
+def decode_pair(elb, spec, seed, n_ctx, walk):
+    """Single-token evaluations at the positions of `walk` (rows in front of them filled by prompt chunks), against the
+    CPU oracle on the same cache contents; every evaluation twice, which must give the same bits."""
+    tens = list(synth.generate(spec, seed))
+    gpu, cpu = elb.Backend(spec, tens, n_ctx), ol.OracleModel(spec, tens, n_ctx)
+    toks = synth.lcg_tokens(n_ctx, spec.n_vocab, seed)
+    filled, worst = 0, 0.0
+    for pos in walk:
+        if pos > filled:
+            gpu.eval(toks[filled:pos], filled, want_logits=False)
+            cpu.eval(toks[filled:pos], filled)
+            filled = pos
+        a, b = gpu.eval(toks[pos:pos + 1], pos), cpu.eval(toks[pos:pos + 1], pos)
+        assert gpu.last_eval_stats()[1] == 1, "the persistent kernel must run"
+        assert np.array_equal(a, gpu.eval(toks[pos:pos + 1], pos)), "deterministic"
+        worst = max(worst, float(np.abs(a - b).max() / np.abs(b).max()))
+        filled = max(filled, pos + 1)
+    gpu.close()
+    cpu.close()
+    return worst
+
+
+# attention splits of 60 keys: one, two, many, back to one, many again (stale partial results must not be taken); every
+# group size of query heads the kernel is compiled for; all-F16 and quantized weights; an odd number of layers
+@pytest.mark.parametrize("layout,heads,kv", (("q4_k_m", 8, 4), ("f16", 6, 2), ("q8_0", 8, 1), ("q6_k", 2, 2)))
+def test_decode_across_attention_splits(elb, layout, heads, kv):
+    spec = synth.Spec(name="small", n_layer=3, n_embd=512, n_ff=768, n_head=heads, n_head_kv=kv, n_vocab=1111, layout=layout,
+                      head_sigma=2e-5)
+    assert decode_pair(elb, spec, 31, 700, (0, 59, 60, 61, 650, 3, 651, 120)) <= 2e-4
+
+
+# a feed-forward vector whose limbs do not fit in shared memory beside the weight rings: worked off in parts along k
+def test_decode_long_feed_forward(elb):
+    spec = synth.Spec(name="small", n_layer=2, n_embd=256, n_ff=25600, n_head=2, n_head_kv=1, n_vocab=640, layout="q4_k_m",
+                      head_sigma=2e-5)
+    assert decode_pair(elb, spec, 32, 80, (0, 17, 70)) <= 2e-4
