@@ -248,14 +248,10 @@ int gemm_f16_launch(const Weight* w, const float* d_x, int64_t ldx, const float*
                     int64_t ldy, const float* d_resid, int epilogue, cudaStream_t s);
 // gemm_f16_tc.cu - tcgen05 path for F16 weights and for Q8_0 weights held as fp16 pairs: the token rows are split into
 // fp16 hi / lo halves (d_scratch: 4 * B * n bytes) with 2^-k per row in d_inv_scale, then one tensor-core GEMM with fp32
-// accumulators in tensor memory. d_part (gemm_f16_tc_part_bytes() bytes) and d_counters (gemm_f16_tc_counters() zeroed
-// words) let a matrix of few tiles be cut along k over more CTAs; null: no cut.
+// accumulators in tensor memory
 bool gemm_f16_tc_usable(const Weight* w, int B);
-size_t gemm_f16_tc_part_bytes();
-int gemm_f16_tc_counters();
 int gemm_f16_tc_launch(const Weight* w, const float* d_x, int64_t ldx, const float* d_norm_w, float eps, int B, void* d_scratch,
-                       float* d_inv_scale, float* d_y, int64_t ldy, const float* d_resid, int epilogue, cudaStream_t s, bool pdl,
-                       float* d_part = nullptr, unsigned* d_counters = nullptr);
+                       float* d_inv_scale, float* d_y, int64_t ldy, const float* d_resid, int epilogue, cudaStream_t s, bool pdl);
 int gemm_f16_tc_check();
 int gemm_f16_tc_wait_expiry(cudaStream_t s);  // test hook: a bounded wait that must run out
 

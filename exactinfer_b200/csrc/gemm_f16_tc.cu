@@ -8,14 +8,17 @@
 // contributes Whi * hi + Whi * lo + Wlo * hi (Wlo * lo is 2^-22 of the product and left out), so that the block scale
 // travels inside the operand and a row's 32-value blocks accumulate in one pass.
 //
-// Few output tiles (a 64-row batch against a 2048-row matrix is 16 tiles for 148 SMs): the k range of a tile is cut
-// into splits that different CTAs accumulate; each leaves its fp32 partial tile in scratch memory and the CTA that
-// arrives last adds the partial tiles in split order, so the result does not depend on which CTA that was.
+// Few output tiles (a 64-row batch against a 2048-row matrix is 16 tiles for 148 SMs): the k range of a tile is cut over
+// the CTAs of a cluster; each leaves its fp32 partial tile in its own shared memory, and every CTA adds a slice of the
+// tokens over all of them through distributed shared memory, in a fixed order. (Partial tiles in L2, added by the CTA that
+// arrived last, took 30-50 us per launch of a 77-row batch: one SM read up to twelve 64 KB tiles, a chain of round trips.)
 //
-// Warp roles (192 threads): warps 0-3 epilogue (warp w drains TMEM lanes 32w.. = weight rows), warp 4 TMA producer,
-// warp 5 MMA issuer and TMEM owner. Operands arrive by TMA into a ring of 128-byte-swizzled K-major
-// tiles (64 k per stage); two accumulators, so that the drain of one tile overlaps the MMAs of the next. A persistent
-// grid walks the output tiles. Every mbarrier wait is bounded: on timeout the kernel raises an error word and winds down.
+// Warp roles: warps 0 .. 4 T/32 - 1 epilogue (warp w drains TMEM lanes 32 (w % 4) .. = weight rows, tokens 32 (w / 4) ..),
+// then one warp as TMA producer and one as MMA issuer and TMEM owner. A thread accumulates 32 tokens of one row: the code
+// of a tile is then short enough not to be bound by its own fetching (one warp per 32 rows with all 128 tokens, unrolled,
+// was). Operands arrive by TMA into a ring of 128-byte-swizzled K-major tiles (64 k per stage); two accumulators, so that
+// the drain of one segment overlaps the MMAs of the next. Without a cut along k a persistent grid walks the output tiles.
+// Every mbarrier wait is bounded: on timeout the kernel raises an error word and winds down.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -28,7 +31,8 @@ namespace elb {
 
 namespace {
 
-constexpr int FT_ROWS = 128, FT_K = 64, FT_THREADS = 192;
+constexpr int FT_ROWS = 128, FT_K = 64;
+constexpr int FT_MAXSPLIT = 8;  // CTAs of a cluster
 constexpr int FT_SEG = 2;  // k tiles (of 64) accumulated in tensor memory before the sum moves to registers
 constexpr unsigned FT_SPIN_LIMIT = 1u << 24;
 
@@ -78,17 +82,15 @@ __device__ __forceinline__ void f_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t
 __device__ __forceinline__ void f_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(f_smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void f_tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
+__device__ __forceinline__ void f_tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ void f_tmem_ld32(uint32_t taddr, float (&v)[32]) {
     uint32_t r[32];
@@ -140,30 +142,72 @@ struct FtParams {
     int64_t rows16, rows, ldy;
     int B, n, epilogue;
     int row_tiles, tok_tiles;
-    int splits;          // k splits per output tile
-    float* part;         // [tile][split][128 rows][T] partial tiles (splits > 1)
-    unsigned* counters;  // [tile] arrivals; the last arrival reduces and zeroes its counter
+    int splits;          // CTAs of a cluster = cuts of k (1: none)
     int* err;
 };
 
 template <int T, bool WLO> struct FtShape {
+    static constexpr int EPI_WARPS = 4 * (T / 32);
+    static constexpr int THREADS = 32 * (EPI_WARPS + 2);
     static constexpr int A_BYTES = FT_ROWS * 128;  // 128 rows x 64 halves (once more for the lo half of a Q8_0 weight)
     static constexpr int B_BYTES = T * 128;        // T tokens x 64 halves, once for hi and once for lo
     static constexpr int STAGE = (WLO ? 2 : 1) * A_BYTES + 2 * B_BYTES;
     static constexpr int STAGES = (200 * 1024) / STAGE > 6 ? 6 : (200 * 1024) / STAGE;
     static constexpr int SMEM = STAGES * STAGE + 256 + 1024;
+    static_assert(STAGES * STAGE >= T * FT_ROWS * 4, "a partial tile takes the place of the operand ring");
     static constexpr int TMEM_COLS = 4 * T;  // two accumulators and the finished tile (3 T columns; a power of two)
 };
 
-// k tiles [k0, k1) of split s of a tile
-__device__ __forceinline__ void ft_k_range(int nk, int splits, int s, int& k0, int& k1) {
-    k0 = int(int64_t(nk) * s / splits);
-    k1 = int(int64_t(nk) * (s + 1) / splits);
+__device__ __forceinline__ uint32_t f_cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void f_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float f_cluster_ld(uint32_t saddr, uint32_t rank) {  // a word of CTA `rank`'s shared memory
+    float v;
+    asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %1, %2;\n ld.shared::cluster.f32 %0, [a];\n}\n"
+                 : "=f"(v) : "r"(saddr), "r"(rank) : "memory");
+    return v;
+}
+
+// N finished tokens tok0 .. of row R (a warp holds 32 consecutive rows): scale, epilogue, store. Every load before the
+// first store: Y may be the residual stream itself, and a load that has to wait for the store before it turns the tokens
+// into a chain of memory round trips.
+template <int N>
+__device__ __forceinline__ void ft_store(const FtParams& p, const float (&v)[N], int tok0, int step, int tok_end, int64_t R, int lane) {
+    float sc[N], r[N];
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+        const int tok = tok0 + t * step;
+        const bool on = tok < tok_end;
+        sc[t] = on ? __ldcg(p.inv_scale + tok) : 0.f;
+        r[t] = p.epilogue == EPI_ADD && on && R < p.rows ? __ldcg(p.resid + int64_t(tok) * p.ldy + R) : 0.f;
+    }
+    if (p.epilogue == EPI_SILU) {  // tile rows 0..7 gate, 8..15 up (16-row groups): partner is 8 lanes up
+        const int64_t o = R / 16 * 8 + (R & 7);
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+            const float y = v[t] * sc[t], up = __shfl_down_sync(0xffffffffu, y, 8);
+            const int tok = tok0 + t * step;
+            if (tok < tok_end && (lane & 8) == 0 && o < p.rows / 2)
+                p.Y[int64_t(tok) * p.ldy + o] = __fmul_rn(__fdiv_rn(y, 1.0f + expf(-y)), up);
+        }
+        return;
+    }
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+        const int tok = tok0 + t * step;
+        const float y = v[t] * sc[t];
+        if (tok < tok_end && R < p.rows) p.Y[int64_t(tok) * p.ldy + R] = p.epilogue == EPI_ADD ? r[t] + y : y;
+    }
 }
 
 template <int T, bool WLO>
-__global__ void __launch_bounds__(FT_THREADS, 1) k_gemm_f16_tc(const __grid_constant__ CUtensorMap mapW,
-                                                               const __grid_constant__ CUtensorMap mapX, const FtParams p) {
+__global__ void __launch_bounds__(FtShape<T, WLO>::THREADS, 1) k_gemm_f16_tc(const __grid_constant__ CUtensorMap mapW,
+                                                                             const __grid_constant__ CUtensorMap mapX, const FtParams p) {
     using S = FtShape<T, WLO>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -173,15 +217,17 @@ __global__ void __launch_bounds__(FT_THREADS, 1) k_gemm_f16_tc(const __grid_cons
     uint64_t* tfull = bars + 2 * S::STAGES;    // [2] MMA -> epilogue
     uint64_t* tempty = tfull + 2;              // [2] epilogue -> MMA
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
-    unsigned* last_slot = tmem_slot + 1;  // split mode: non-zero when this CTA is the tile's last arrival
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nk = p.n / FT_K, n_items = p.row_tiles * p.tok_tiles * p.splits;  // item = tile * splits + split
+    const int nk = p.n / FT_K, n_tiles = p.row_tiles * p.tok_tiles;
+    // cluster c works on output tiles c, c + clusters, ... (with a cut along k: on tile c alone)
+    const int split = p.splits > 1 ? int(f_cluster_rank()) : 0, tile0 = blockIdx.x / p.splits, tile_step = gridDim.x / p.splits;
+    const int k0 = nk * split / p.splits, k1 = nk * (split + 1) / p.splits;
     if (tid == 0) {
         for (int s = 0; s < S::STAGES; ++s) { f_mbar_init(full + s, 1); f_mbar_init(empty + s, 1); }
-        for (int a = 0; a < 2; ++a) { f_mbar_init(tfull + a, 1); f_mbar_init(tempty + a, 4); }
+        for (int a = 0; a < 2; ++a) { f_mbar_init(tfull + a, 1); f_mbar_init(tempty + a, S::EPI_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 5) {
+    if (warp == S::EPI_WARPS + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(f_smem_u32(tmem_slot)), "n"(S::TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -192,14 +238,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) k_gemm_f16_tc(const __grid_cons
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
 
-    if (warp == 4) {
+    if (warp == S::EPI_WARPS) {
         if (lane == 0) {  // ---- TMA producer
             int it = 0;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const int tile = item / p.splits;
+            for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
                 const int row0 = tile / p.tok_tiles * FT_ROWS, tok0 = tile % p.tok_tiles * T;
-                int k0, k1;
-                ft_k_range(nk, p.splits, item % p.splits, k0, k1);
                 for (int kt = k0; kt < k1 && ok; ++kt, ++it) {
                     const int s = it % S::STAGES;
                     ok = f_mbar_wait(empty + s, ((it / S::STAGES) & 1) ^ 1);
@@ -218,13 +261,11 @@ __global__ void __launch_bounds__(FT_THREADS, 1) k_gemm_f16_tc(const __grid_cons
                 }
             }
         }
-    } else if (warp == 5) {
+    } else if (warp == S::EPI_WARPS + 1) {
         if (lane == 0) {  // ---- MMA issuer
             constexpr uint32_t idesc = f_idesc(FT_ROWS, T);
             int it = 0, ns = 0;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                int k0, k1;
-                ft_k_range(nk, p.splits, item % p.splits, k0, k1);
+            for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
                 for (int ks0 = k0; ks0 < k1 && ok; ks0 += FT_SEG, ++ns) {  // one segment into one accumulator
                     const int acc = ns & 1, ks1 = min(ks0 + FT_SEG, k1);
                     ok = f_mbar_wait(tempty + acc, ((ns >> 1) & 1) ^ 1);  // the accumulator has been drained
@@ -249,129 +290,79 @@ __global__ void __launch_bounds__(FT_THREADS, 1) k_gemm_f16_tc(const __grid_cons
                 }
             }
         }
-    } else {  // ---- epilogue: warp w drains TMEM lanes 32w.. (weight rows), all T tokens
+    } else {  // ---- epilogue
+        const uint32_t tlane = uint32_t((warp & 3) * 32) << 16;
+        const int c0 = (warp >> 2) * 32;
         int ns = 0;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const int tile = item / p.splits;
+        for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
             const int row0 = tile / p.tok_tiles * FT_ROWS, tok0 = tile % p.tok_tiles * T;
-            const int64_t R = row0 + warp * 32 + lane;
-            int k0, k1;
-            ft_k_range(nk, p.splits, item % p.splits, k0, k1);
             // The tensor core adds into its fp32 accumulator with truncation, a bias that grows with the length of the
             // chain: a segment of FT_SEG k tiles is accumulated there, the segments are added here with rounding.
-            float accf[T];
+            float acc[32];
 #pragma unroll
-            for (int i = 0; i < T; ++i) accf[i] = 0.f;
+            for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+#pragma unroll 1
             for (int ks0 = k0; ks0 < k1 && ok; ks0 += FT_SEG, ++ns) {
-                const int acc = ns & 1;
-                ok = f_mbar_wait(tfull + acc, (ns >> 1) & 1);
+                const int a = ns & 1;
+                ok = f_mbar_wait(tfull + a, (ns >> 1) & 1);
                 if (!ok) break;
                 f_fence_after();
-                const uint32_t tbase = tmem_base + acc * T + (uint32_t(warp * 32) << 16);
+                float v[32];
+                f_tmem_ld32(tmem_base + a * T + c0 + tlane, v);
 #pragma unroll
-                for (int c = 0; c < T; c += 32) {
-                    float v[32];
-                    f_tmem_ld32(tbase + c, v);
-#pragma unroll
-                    for (int t = 0; t < 32; ++t) accf[c + t] += v[t];
-                }
+                for (int t = 0; t < 32; ++t) acc[t] += v[t];
                 f_fence_before();  // accumulator in registers: the issuer may overwrite it
                 __syncwarp();
-                if (lane == 0) f_mbar_arrive(tempty + acc);
+                if (lane == 0) f_mbar_arrive(tempty + a);
             }
             if (!ok) break;
-            if (p.splits > 1) {
-                float* dst = p.part + (size_t(item) * FT_ROWS + warp * 32 + lane) * T;
+            if (p.splits > 1) {  // the partial tile -> this CTA's shared memory [token][row] (the operand ring is used up)
+                float* part = reinterpret_cast<float*>(smem) + c0 * FT_ROWS + (warp & 3) * 32 + lane;
 #pragma unroll
-                for (int t = 0; t < T; t += 4) __stcg(reinterpret_cast<float4*>(dst + t), make_float4(accf[t], accf[t + 1], accf[t + 2], accf[t + 3]));
-                __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps
-                if (tid == 0) {
-                    const unsigned seen = atomicAdd(p.counters + tile, 1u);
-                    *last_slot = seen == unsigned(p.splits - 1);
-                    if (seen == unsigned(p.splits - 1)) p.counters[tile] = 0;  // ready for the next launch
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                const bool last = *last_slot != 0;
-                asm volatile("bar.sync 1, 128;" ::: "memory");  // everyone has read the slot before the next item writes it
-                if (!last) continue;
-                __threadfence();
-                // the partial tiles in split order, whichever CTA came last (its own included, read back like the others)
-                const float* mine = p.part + (size_t(tile) * p.splits * FT_ROWS + warp * 32 + lane) * T;
-#pragma unroll
-                for (int t = 0; t < T; t += 4) {
-                    const float4 a = __ldcg(reinterpret_cast<const float4*>(mine + t));
-                    accf[t] = a.x; accf[t + 1] = a.y; accf[t + 2] = a.z; accf[t + 3] = a.w;
-                }
-                // (32 tokens of two partial tiles are requested before the first of them is added: the loop is a chain
-                // of round trips to L2 otherwise; the order of the additions stays split 1, 2, 3, ...)
-                for (int s2 = 1; s2 < p.splits; s2 += 2) {
-                    const float* q0 = mine + size_t(s2) * FT_ROWS * T;
-                    const bool two = s2 + 1 < p.splits;
-                    const float* q1 = two ? q0 + size_t(FT_ROWS) * T : q0;
-#pragma unroll
-                    for (int c = 0; c < T; c += 32) {
-                        float4 a[8], b[8];
-#pragma unroll
-                        for (int t = 0; t < 8; ++t) {
-                            a[t] = __ldcg(reinterpret_cast<const float4*>(q0 + c) + t);
-                            b[t] = __ldcg(reinterpret_cast<const float4*>(q1 + c) + t);
-                        }
-#pragma unroll
-                        for (int t = 0; t < 8; ++t) {
-                            accf[c + 4 * t] += a[t].x; accf[c + 4 * t + 1] += a[t].y; accf[c + 4 * t + 2] += a[t].z; accf[c + 4 * t + 3] += a[t].w;
-                        }
-                        if (two) {
-#pragma unroll
-                            for (int t = 0; t < 8; ++t) {
-                                accf[c + 4 * t] += b[t].x; accf[c + 4 * t + 1] += b[t].y; accf[c + 4 * t + 2] += b[t].z; accf[c + 4 * t + 3] += b[t].w;
-                            }
-                        }
-                    }
-                }
+                for (int t = 0; t < 32; ++t) part[t * FT_ROWS] = acc[t];
+                break;
             }
-            // The finished tile goes back to tensor memory, from where a compact loop writes it out 32 tokens at a
-            // time (a loop over the register array would have to be unrolled: code that runs once per tile, straight
-            // from instruction memory).
-            const uint32_t tdone = tmem_base + 2 * T + (uint32_t(warp * 32) << 16);
-#pragma unroll
-            for (int c = 0; c < T; c += 32) f_tmem_st32(tdone + c, *reinterpret_cast<const float(*)[32]>(&accf[c]));
+            // The finished tile goes back to tensor memory, from where a rolled loop writes it out 8 tokens at a time (a
+            // loop over the register array would have to be unrolled: code that runs once per tile).
+            const uint32_t tdone = tmem_base + 2 * T + c0 + tlane;
+            f_tmem_st32(tdone, acc);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 #pragma unroll 1
-            for (int c = 0; c < T; c += 32) {
-                float v[32];
-                f_tmem_ld32(tdone + c, v);
-                // every load of the 32 tokens before the first store: Y may be the residual stream itself, and a load
-                // that has to wait for the store before it turns the chunk into a chain of memory round trips
-                float sc[32], r[32];
-#pragma unroll
-                for (int t = 0; t < 32; ++t) {
-                    const int tok = tok0 + c + t;
-                    sc[t] = tok < p.B ? __ldcg(p.inv_scale + tok) : 0.f;
-                    r[t] = p.epilogue == EPI_ADD && tok < p.B && R < p.rows ? __ldcg(p.resid + int64_t(tok) * p.ldy + R) : 0.f;
-                }
-#pragma unroll
-                for (int t = 0; t < 32; ++t) {
-                    const int tok = tok0 + c + t;
-                    const bool tok_ok = tok < p.B;
-                    const float y = v[t] * sc[t];
-                    if (p.epilogue == EPI_SILU) {  // tile rows 0..7 gate, 8..15 up (16-row groups): partner is 8 lanes up
-                        const float up = __shfl_down_sync(0xffffffffu, y, 8);
-                        const int64_t o = R / 16 * 8 + (R & 7);
-                        if (tok_ok && (lane & 8) == 0 && o < p.rows / 2)
-                            p.Y[int64_t(tok) * p.ldy + o] = __fmul_rn(__fdiv_rn(y, 1.0f + expf(-y)), up);
-                    } else if (tok_ok && R < p.rows) {
-                        p.Y[int64_t(tok) * p.ldy + R] = p.epilogue == EPI_ADD ? r[t] + y : y;
-                    }
-                }
+            for (int c = 0; c < 32; c += 8) {
+                if (tok0 + c0 + c >= p.B) break;
+                float v[8];
+                f_tmem_ld8(tdone + c, v);
+                ft_store<8>(p, v, tok0 + c0 + c, 1, min(tok0 + c0 + c + 8, p.B), row0 + (warp & 3) * 32 + lane, lane);
             }
         }
     }
     if (!ok) atomicExch(p.err, 3);
+    if (p.splits > 1) {
+        __syncwarp();
+        f_cluster_sync();
+        if (warp < S::EPI_WARPS && tile0 < n_tiles) {
+            // this CTA's slice of the tile's tokens, summed over the cluster in rank order; a warp takes every (T / 32)-th token
+            const int row0 = tile0 / p.tok_tiles * FT_ROWS, tok0 = tile0 % p.tok_tiles * T, tn = min(T, p.B - tok0);
+            const int lo = tn * split / p.splits, hi = tn * (split + 1) / p.splits, r = (warp & 3) * 32 + lane;
+            const uint32_t base = f_smem_u32(smem) + uint32_t(r) * 4u;
+            constexpr int G = T / 32;
+#pragma unroll 1
+            for (int t = lo + (warp >> 2); t < hi; t += 4 * G) {
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+                for (int q = 0; q < p.splits; ++q)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (t + j * G < hi) v[j] += f_cluster_ld(base + uint32_t(t + j * G) * (FT_ROWS * 4), uint32_t(q));
+                ft_store<4>(p, v, tok0 + t, G, tok0 + hi, row0 + r, lane);
+            }
+        }
+        f_cluster_sync();  // nobody leaves while its shared memory is being read
+    }
     pdl_launch_dependents();
     f_fence_before();
     __syncthreads();
-    if (warp == 5) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(S::TMEM_COLS) : "memory");
+    if (warp == S::EPI_WARPS + 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(S::TMEM_COLS) : "memory");
 }
 
 // The kernel's bounded wait on a barrier that nobody arrives at (a short limit): it must give up, raise the error word
@@ -526,14 +517,9 @@ int gemm_f16_tc_check() {  // after a synchronize: did the kernel give up on a w
     return ELB_OK;
 }
 
-size_t gemm_f16_tc_part_bytes() { return size_t(2) * 148 * FT_ROWS * 128 * sizeof(float); }  // two items per SM at T = 128
-int gemm_f16_tc_counters() { return 4096; }
-
-// scratch: room for hi and lo, 2 * B * n halves (the model's limb buffer has exactly that size). d_part / d_counters:
-// gemm_f16_tc_part_bytes() bytes and gemm_f16_tc_counters() zeroed words for the k splits, or null (no splits).
+// scratch: room for hi and lo, 2 * B * n halves (the model's limb buffer has exactly that size)
 int gemm_f16_tc_launch(const Weight* w, const float* d_x, int64_t ldx, const float* d_norm_w, float eps, int B, void* d_scratch,
-                       float* d_inv_scale, float* d_y, int64_t ldy, const float* d_resid, int epilogue, cudaStream_t s, bool pdl,
-                       float* d_part, unsigned* d_counters) {
+                       float* d_inv_scale, float* d_y, int64_t ldy, const float* d_resid, int epilogue, cudaStream_t s, bool pdl) {
     if (!gemm_f16_tc_usable(w, B)) return fail(ELB_ERR_STATE, "matmul: F16 tensor-core path not usable for this weight");
     if (epilogue == EPI_SILU && !w->pair) return fail(ELB_ERR_INVALID, "matmul: SwiGLU epilogue needs a paired weight");
     int* err_host = f_error_word();
@@ -565,35 +551,36 @@ int gemm_f16_tc_launch(const Weight* w, const float* d_x, int64_t ldx, const flo
     DeviceInfo di;
     ELB_TRY(device_info(w->device, &di));
     const int64_t tiles = int64_t(row_tiles) * tok_tiles;
-    int splits = 1;
-    static const int max_splits = [] { const char* v = std::getenv("ELB_TC_SPLITS"); return v ? std::max(1, atoi(v)) : 16; }();
-    if (d_part && d_counters && tiles < di.sm_count && tiles <= gemm_f16_tc_counters()) {
-        splits = int(std::min<int64_t>({int64_t(di.sm_count) / tiles, int64_t(n / FT_K / 4), int64_t(max_splits)}));
-        splits = std::max(splits, 1);
-        while (splits > 1 && size_t(tiles) * splits * FT_ROWS * T * sizeof(float) > gemm_f16_tc_part_bytes()) --splits;
-    }
-    FtParams p{d_inv_scale, d_y, d_resid, rows16, w->rows, ldy, B, n, epilogue, row_tiles, tok_tiles, splits, d_part, d_counters, err_dev};
-    const int grid = int(std::min<int64_t>(tiles * splits, di.sm_count));
-    auto launch = [&](auto kernel, int smem) -> int {
+    // fewer tiles than SMs: k is cut over a cluster, as long as every CTA keeps two k tiles (one segment)
+    static const int max_splits = [] { const char* v = std::getenv("ELB_TC_SPLITS"); return v ? std::max(1, atoi(v)) : FT_MAXSPLIT; }();
+    const int splits = int(std::max<int64_t>(1, std::min<int64_t>({int64_t(di.sm_count) / tiles, int64_t(n / FT_K / FT_SEG), int64_t(std::min(max_splits, FT_MAXSPLIT))})));
+    FtParams p{d_inv_scale, d_y, d_resid, rows16, w->rows, ldy, B, n, epilogue, row_tiles, tok_tiles, splits, err_dev};
+    const int grid = int(splits > 1 ? tiles * splits : std::min<int64_t>(tiles, di.sm_count));
+    auto launch = [&](auto kernel, int smem, int threads) -> int {
         ELB_TRY(ensure_dyn_smem(reinterpret_cast<const void*>(kernel), size_t(smem)));
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(unsigned(grid));
-        cfg.blockDim = dim3(FT_THREADS);
+        cfg.blockDim = dim3(unsigned(threads));
         cfg.dynamicSmemBytes = size_t(smem);
         cfg.stream = s;
-        cfg.attrs = attr;
-        cfg.numAttrs = pdl ? 1 : 0;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = unsigned(splits);
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        at[1] = attr[0];
+        cfg.attrs = at;
+        cfg.numAttrs = pdl ? 2 : 1;
         ELB_CUDA(cudaLaunchKernelEx(&cfg, kernel, mapW, mapX, p));
         return ELB_OK;
     };
     if (wlo) {
-        if (T == 128) ELB_TRY(launch(k_gemm_f16_tc<128, true>, FtShape<128, true>::SMEM));
-        else if (T == 64) ELB_TRY(launch(k_gemm_f16_tc<64, true>, FtShape<64, true>::SMEM));
-        else ELB_TRY(launch(k_gemm_f16_tc<32, true>, FtShape<32, true>::SMEM));
+        if (T == 128) ELB_TRY(launch(k_gemm_f16_tc<128, true>, FtShape<128, true>::SMEM, FtShape<128, true>::THREADS));
+        else if (T == 64) ELB_TRY(launch(k_gemm_f16_tc<64, true>, FtShape<64, true>::SMEM, FtShape<64, true>::THREADS));
+        else ELB_TRY(launch(k_gemm_f16_tc<32, true>, FtShape<32, true>::SMEM, FtShape<32, true>::THREADS));
     } else {
-        if (T == 128) ELB_TRY(launch(k_gemm_f16_tc<128, false>, FtShape<128, false>::SMEM));
-        else if (T == 64) ELB_TRY(launch(k_gemm_f16_tc<64, false>, FtShape<64, false>::SMEM));
-        else ELB_TRY(launch(k_gemm_f16_tc<32, false>, FtShape<32, false>::SMEM));
+        if (T == 128) ELB_TRY(launch(k_gemm_f16_tc<128, false>, FtShape<128, false>::SMEM, FtShape<128, false>::THREADS));
+        else if (T == 64) ELB_TRY(launch(k_gemm_f16_tc<64, false>, FtShape<64, false>::SMEM, FtShape<64, false>::THREADS));
+        else ELB_TRY(launch(k_gemm_f16_tc<32, false>, FtShape<32, false>::SMEM, FtShape<32, false>::THREADS));
     }
     ELB_CUDA(cudaGetLastError());
     return ELB_OK;

@@ -55,8 +55,6 @@ struct Model {
     int8_t* limbs = nullptr;
     float *inv_scale = nullptr, *xsum = nullptr;
     void* kv16 = nullptr;             // keys and values of one layer as fp16 pairs (tensor-core prompt attention)
-    float* tc_part = nullptr;         // partial tiles and arrival counters of the fp16 tensor-core GEMM's k splits
-    unsigned* tc_counters = nullptr;
     int32_t* tokens_dev = nullptr;
     int* pos_dev = nullptr;
     int32_t* tokens_host = nullptr;  // pinned
@@ -197,8 +195,7 @@ int linear_tokens(Model* m, const Weight* w, const float* xin, int64_t ldx, cons
     ++m->launches;
     if (gemm_f16_tc_usable(w, B)) {  // F16, and Q8_0 held as fp16 pairs
         ++m->launches;  // the hi / lo split of the rows
-        return gemm_f16_tc_launch(w, xin, ldx, norm_w, m->cfg.eps, B, m->limbs, m->inv_scale, y, ldy, resid, epi, m->stream, m->use_pdl,
-                                  m->tc_part, m->tc_counters);
+        return gemm_f16_tc_launch(w, xin, ldx, norm_w, m->cfg.eps, B, m->limbs, m->inv_scale, y, ldy, resid, epi, m->stream, m->use_pdl);
     }
     if (w->type == ELB_F16) return gemm_f16_launch(w, xin, ldx, norm_w, m->cfg.eps, B, y, ldy, resid, epi, m->stream);
     if (gemm_tc_usable(w, B)) return gemm_tc_launch(w, m->limbs, m->inv_scale, m->xsum, B, nl, y, ldy, resid, epi, m->stream, m->use_pdl);
@@ -900,7 +897,7 @@ void model_destroy(Model* m) {
                     (void*)m->tokens_dev, (void*)m->pos_dev, (void*)m->attn_part, (void*)m->attn_counters, (void*)m->dlimbs[0],
                     (void*)m->dlimbs[1], (void*)m->dlimbs[2], (void*)m->dlimbs[3], (void*)m->dinv, (void*)m->done})
         cudaFree(p);
-    cudaFree(m->exchange); cudaFree(m->f16_maps); cudaFree(m->xbuf); cudaFree(m->xctl); cudaFree(m->gact); cudaFree(m->tc_part); cudaFree(m->tc_counters); cudaFree(m->kv16);
+    cudaFree(m->exchange); cudaFree(m->f16_maps); cudaFree(m->xbuf); cudaFree(m->xctl); cudaFree(m->gact); cudaFree(m->kv16);
     if (m->xarea.local) tp_peer_free(&m->xarea, m->tp.rank); cudaFree(m->sync_words); cudaFree(m->pos_steps);
     cudaFree(m->xr); cudaFree(m->logits_local);
     cudaFree(m->ap_part); cudaFree(m->ap_counters); cudaFree(m->top_dev); cudaFree(m->mask_dev);
@@ -1063,9 +1060,6 @@ static int finalize_local(Model* m) {
     }
     ELB_CUDA(cudaMalloc(&m->limbs, size_t(4) * B * maxn));
     ELB_CUDA(cudaMalloc(&m->inv_scale, size_t(B) * 4));
-    ELB_CUDA(cudaMalloc(&m->tc_part, gemm_f16_tc_part_bytes()));
-    ELB_CUDA(cudaMalloc(&m->tc_counters, size_t(gemm_f16_tc_counters()) * sizeof(unsigned)));
-    ELB_CUDA(cudaMemset(m->tc_counters, 0, size_t(gemm_f16_tc_counters()) * sizeof(unsigned)));
     ELB_CUDA(cudaMalloc(&m->xsum, size_t(B) * (maxn / 32 + 1) * 4));
     ELB_CUDA(cudaMalloc(&m->tokens_dev, size_t(B) * sizeof(int32_t)));
     ELB_CUDA(cudaMalloc(&m->pos_dev, sizeof(int)));
