@@ -15,6 +15,11 @@
 // fragments. The three products of every step are a chain of their own, started from zero, and join the running score or
 // output in fp32 registers with rounding (the tensor core's own accumulation truncates toward zero). Keys are cut into chunks per query tile with
 // the same partial-result layout and last-arrival combination as k_attn_prefill_gqa (deterministic chunk order).
+// A tile of 64 keys takes a CTA 6 us or more, a serial chain of loads, MMAs and exponentials: what bounds a launch is how
+// many tiles the longest CTA walks. The cut therefore follows the launch (attn_prefill_tc_launch) and the full chunks go
+// first. With 256 keys per chunk at least, and short chunks first, 77 rows behind 203 took 38 us on 40 CTAs, 2 rows behind
+// 2048 41 us on 56; a 77-token turn of the 0.6B shape went from 3.32 to 3.03 ms, a 2050-token prompt of the 1.7B shape from
+// 41.1 to 38.3 ms, 512 tokens of the 4B shape from 21.87 to 21.65 ms.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -27,7 +32,9 @@ namespace elb {
 namespace {
 
 constexpr int D = 128;
-constexpr int AT_ROWS = 64, AT_K = 64, AT_THREADS = 128, AT_MAXCHUNK = 8;
+constexpr int AT_ROWS = 64, AT_K = 64, AT_THREADS = 128;
+constexpr int AT_SCRATCH_CHUNKS = 8;  // partial results per query tile of a full batch that the scratch has room for
+constexpr int AT_MAXCHUNK = 24;       // chunks of one query tile (the last to arrive adds them one after the other)
 constexpr int AT_LDK = D + 8;      // halves per key row in shared memory: 272 bytes, fragment loads hit 32 banks
 constexpr int AT_LDV = AT_K + 8;   // halves per dimension row of V^T: 144 bytes
 constexpr int AT_PART = AT_ROWS * (D + 2);  // floats per partial result (layout of k_attn_prefill_gqa)
@@ -99,6 +106,7 @@ struct AtParams {
     float* att;
     int64_t ld_att;
     int pos0, B, H, HKV, kchunk;  // kchunk: 64-key tiles per chunk
+    int max_chunk;                // chunks of the longest query tile
     float scale;
     float* part;
     unsigned* counters;
@@ -115,10 +123,11 @@ __global__ void __launch_bounds__(AT_THREADS, 2) k_attn_prefill_tc(const AtParam
     __shared__ int s_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int kvh = blockIdx.x, group = p.H / p.HKV, TQ = AT_ROWS / group, n_qt = (p.B + TQ - 1) / TQ;
-    int qt = 0, chunk = int(blockIdx.y), n_chunks = at_chunks(p.pos0, p.B, TQ, 0, p.kchunk);  // item -> (query tile, chunk)
-    while (chunk >= n_chunks && qt + 1 < n_qt) {
+    // item -> (query tile, chunk), the last query tiles first: theirs are the full chunks, and a short one fits behind them
+    int qt = n_qt - 1, chunk = int(blockIdx.y), n_chunks = at_chunks(p.pos0, p.B, TQ, qt, p.kchunk);
+    while (chunk >= n_chunks && qt > 0) {
         chunk -= n_chunks;
-        ++qt;
+        --qt;
         n_chunks = at_chunks(p.pos0, p.B, TQ, qt, p.kchunk);
     }
     const int q0 = qt * TQ, nq = min(TQ, p.B - q0);
@@ -164,8 +173,10 @@ __global__ void __launch_bounds__(AT_THREADS, 2) k_attn_prefill_tc(const AtParam
     load_k(t_first);
     load_v(t_first);
     // Q as fp16 pairs in shared memory (row r = head * TQ + token), read as A fragments per 16-dimension step
+    const int tq_log2 = 31 - __clz(TQ);  // (a power of two: a group is a divisor of 64)
+#pragma unroll 8
     for (int i = tid; i < AT_ROWS * 64; i += AT_THREADS) {
-        const int r = i >> 6, c = (i & 63) * 2, h = r / TQ, tk = r - h * TQ;
+        const int r = i >> 6, c = (i & 63) * 2, h = r >> tq_log2, tk = r - h * TQ;
         float2 q = make_float2(0.f, 0.f);
         if (tk < nq) q = *reinterpret_cast<const float2*>(p.qkv + int64_t(q0 + tk) * p.ld + (kvh * group + h) * D + c);
         uint32_t hi, lo;
@@ -298,7 +309,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) k_attn_prefill_tc(const AtParam
         o[nt][0] *= 1.0f / AT_PSCALE; o[nt][1] *= 1.0f / AT_PSCALE; o[nt][2] *= 1.0f / AT_PSCALE; o[nt][3] *= 1.0f / AT_PSCALE;
     }
     if (n_chunks > 1) {  // leave this chunk's result; the last chunk of the query tile to arrive adds them all
-        float* base = p.part + (size_t(kvh) * n_qt + qt) * AT_MAXCHUNK * AT_PART;
+        float* base = p.part + (size_t(kvh) * n_qt + qt) * p.max_chunk * AT_PART;
         float* mine = base + size_t(chunk) * AT_PART;
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -365,7 +376,8 @@ bool attn_prefill_tc_usable(int H, int HKV, int64_t ld, int64_t ld_att) {
 
 // part / counters: the scratch of attn_prefill_launch (same sizes); kv16: attn_prefill_tc_scratch_halves(n_ctx, HKV * 128) halves
 int attn_prefill_tc_launch(const float* qkv, int64_t ld, const float* kc, const float* vc, float* att, int64_t ld_att, int pos0,
-                           int B, int H, int HKV, float scale, cudaStream_t s, float* part, unsigned* counters, void* kv16) {
+                           int B, int H, int HKV, float scale, cudaStream_t s, float* part, unsigned* counters, void* kv16, int max_batch,
+                           int sm_count) {
     if (!attn_prefill_tc_usable(H, HKV, ld, ld_att) || !kv16 || !part || !counters)
         return fail(ELB_ERR_STATE, "attention: tensor-core prompt attention not usable here");
     const int T = pos0 + B, Tp = (T + AT_K - 1) / AT_K * AT_K, KD = HKV * D, group = H / HKV, TQ = AT_ROWS / group;
@@ -377,12 +389,28 @@ int attn_prefill_tc_launch(const float* qkv, int64_t ld, const float* kc, const 
     ELB_CUDA(cudaGetLastError());
     ELB_TRY(ensure_dyn_smem(reinterpret_cast<const void*>(k_attn_prefill_tc), AT_SMEM));
     const int n_qt = (B + TQ - 1) / TQ, tiles_max = Tp / AT_K;
-    // chunks of >= 256 keys (a CTA's fixed costs - Q, first tile, partial result - are worth several tiles), at most 8 per query tile
-    static const int min_chunk = [] { const char* v = std::getenv("ELB_ATTN_TC_CHUNK"); return v ? std::max(1, atoi(v)) : 4; }();
-    const int kchunk = std::max(min_chunk, (tiles_max + AT_MAXCHUNK - 1) / AT_MAXCHUNK);
-    int items = 0;
-    for (int i = 0; i < n_qt; ++i) items += at_chunks(pos0, B, TQ, i, kchunk);
-    AtParams p{qkv, ld, kh, kl, vth, vtl, Tp, KD, att, ld_att, pos0, B, H, HKV, kchunk, scale, part, counters};
+    // How many tiles of 64 keys a CTA walks, from what the launch would then take, in tile times (6 us with one CTA on an SM;
+    // two fit): a CTA's share of the work or its longest chunk, half a chunk for the uneven end when there are more CTAs than
+    // places, a tile for the fixed costs (Q, the first tile), and what the last CTA of a query tile spends on the other
+    // chunks' results. The partial results must fit the scratch, which is made for AT_SCRATCH_CHUNKS of a full batch.
+    const int64_t room = int64_t((max_batch + TQ - 1) / TQ) * AT_SCRATCH_CHUNKS;
+    const int most = int(std::min<int64_t>(AT_MAXCHUNK, std::max<int64_t>(1, room / n_qt)));
+    int kchunk = tiles_max, items = n_qt;
+    double best = 0;
+    for (int cut = 1; cut <= std::min(most, tiles_max); ++cut) {
+        const int k = (tiles_max + cut - 1) / cut, chunks = (tiles_max + k - 1) / k;
+        int n = 0;
+        double work = 0;
+        for (int i = 0; i < n_qt; ++i) {
+            const int c = at_chunks(pos0, B, TQ, i, k);
+            n += c;
+            work += double((std::min(B, (i + 1) * TQ) + pos0 + AT_K - 1) / AT_K + c);
+        }
+        const double longest = k + 1, share = work * HKV / (2.0 * sm_count);
+        const double cost = std::max(longest, share) + (int64_t(n) * HKV > 2 * sm_count ? 0.5 * longest : 0.0) + (chunks > 1 ? 0.5 + 0.15 * chunks : 0.0);
+        if (cut == 1 || cost < best) { best = cost; kchunk = k; items = n; }
+    }
+    AtParams p{qkv, ld, kh, kl, vth, vtl, Tp, KD, att, ld_att, pos0, B, H, HKV, kchunk, (tiles_max + kchunk - 1) / kchunk, scale, part, counters};
     k_attn_prefill_tc<<<dim3(HKV, items), AT_THREADS, AT_SMEM, s>>>(p);
     ELB_CUDA(cudaGetLastError());
     return ELB_OK;

@@ -245,7 +245,8 @@ int body_prefill(Model* m, int B, int pos0, int seq0 = 0, const int* posv_host =
         } else {
             ELB_TRY(qkv_post_launch(m->qkv, QKV, L.q_norm, L.k_norm, m->rope, pos0, B, kc, vc, H, HKV, c.rope_dim, c.eps, m->stream));
             if (m->kv16 && attn_prefill_tc_usable(H, HKV, QKV, QD)) {
-                ELB_TRY(attn_prefill_tc_launch(m->qkv, QKV, kc, vc, m->att, QD, pos0, B, H, HKV, scale, m->stream, m->ap_part, m->ap_counters, m->kv16));
+                ELB_TRY(attn_prefill_tc_launch(m->qkv, QKV, kc, vc, m->att, QD, pos0, B, H, HKV, scale, m->stream, m->ap_part, m->ap_counters, m->kv16,
+                                               m->max_batch, m->sm_count));
                 ++m->launches;  // the fp16 split of the layer's keys and values
             } else {
                 ELB_TRY(attn_prefill_launch(m->qkv, QKV, kc, vc, m->att, QD, pos0, B, H, HKV, scale, m->stream, m->ap_part, m->ap_counters));

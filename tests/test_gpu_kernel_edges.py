@@ -110,3 +110,26 @@ def test_decode_long_feed_forward(elb):
     spec = synth.Spec(name="small", n_layer=2, n_embd=256, n_ff=25600, n_head=2, n_head_kv=1, n_vocab=640, layout="q4_k_m",
                       head_sigma=2e-5)
     assert decode_pair(elb, spec, 32, 80, (0, 17, 70)) <= 2e-4
+
+
+# prompt attention: query tiles that are not full, one key tile, cuts of few and of many key tiles (more partial results per
+# query tile than a full batch could have), a cut with a short last chunk, more CTAs than places
+@pytest.mark.parametrize("heads,kv", ((4, 2), (8, 1), (4, 4)))
+@pytest.mark.parametrize("pos0,n", ((0, 2), (63, 2), (0, 65), (203, 77), (1500, 3), (1400, 130), (0, 512)))
+def test_prompt_attention_cuts(elb, heads, kv, pos0, n):
+    """The same tokens in one chunk and in chunks of 64, which cut the keys differently: the order of fp32 sums differs, no more."""
+    spec = synth.Spec(name="small", n_layer=1, n_embd=256, n_ff=512, n_head=heads, n_head_kv=kv, n_vocab=512, layout="q8_0",
+                      head_sigma=1e-4)
+    tens = list(synth.generate(spec, 3))
+    toks = synth.lcg_tokens(pos0 + n, spec.n_vocab)
+    a, b = elb.Backend(spec, tens, 1664), elb.Backend(spec, tens, 1664)
+    if pos0:
+        a.eval(toks[:pos0], 0, want_logits=False)
+        b.eval(toks[:pos0], 0, want_logits=False)
+    got = a.eval(toks[pos0:], pos0)
+    for lo in range(pos0, pos0 + n, 64):
+        want = b.eval(toks[lo:min(lo + 64, pos0 + n)], lo)
+    # scores, probabilities and sums carry 24 bits; fp32 sums over up to 1664 keys in another order: 2^-24 sqrt(1664) of the
+    # values' size, a few such steps in a layer
+    assert np.linalg.norm(got - want) <= 8 * 2.0 ** -24 * np.sqrt(1664) * np.linalg.norm(want)
+    assert np.array_equal(got.view(np.uint32), a.eval(toks[pos0:], pos0).view(np.uint32))
