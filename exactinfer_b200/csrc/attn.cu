@@ -234,6 +234,8 @@ __global__ void __launch_bounds__(256) k_qkv_post(float* qkv, int64_t ld, const 
                                                  int rope_dim, float eps, const int* posv, const int* seqv,
                                                  size_t seq_stride) {
     const int b = blockIdx.x, hd = blockIdx.y * 8 + threadIdx.y, lane = threadIdx.x, QD = H * D, KD = HKV * D;
+    pdl_launch_dependents();
+    pdl_wait();
     if (hd >= H + 2 * HKV) return;  // (warps only: nothing below synchronises the block)
     const int pos = posv ? posv[b] : pos0 + b;
     if (seqv) { kc += size_t(seqv[b]) * seq_stride; vc += size_t(seqv[b]) * seq_stride; }
@@ -560,6 +562,7 @@ __global__ void __launch_bounds__(AR_THREADS, 2) k_attn_rows(const AttnRowsParam
     __shared__ int s_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int b = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, group = p.H / p.HKV, KD = p.HKV * D;
+    pdl_wait();
     const int T = p.posv[b] + 1, ns = min(p.nsplit, (T + p.per_split - 1) / p.per_split);
     if (split >= ns) return;
     const float* kc = p.kc + size_t(p.seqv[b]) * p.seq_stride + kvh * D;
@@ -619,7 +622,7 @@ size_t attn_rows_part_floats(int H) { return size_t(AR_ROW_SPLITS) * H * (D + 2)
 // posv_host: the rows' positions on the host (they decide how the keys are cut)
 int attn_rows_launch(const float* qkv, int64_t ld, const float* kc, const float* vc, size_t seq_stride, const int* posv,
                      const int* seqv, const int* posv_host, float* att, int64_t ld_att, float* part, unsigned* counters, int B, int H,
-                     int HKV, float scale, int sm_count, cudaStream_t s) {
+                     int HKV, float scale, int sm_count, cudaStream_t s, bool pdl) {
     if (H % HKV || H / HKV > AD_MAXG) return fail(ELB_ERR_UNSUPPORTED, "attention: at most 8 query heads per KV head");
     // Ranges of 256 keys, halved (down to 64: below that the fixed cost of a CTA and of the combination outweighs its keys)
     // until the GPU has two CTAs per SM.
@@ -637,11 +640,7 @@ int attn_rows_launch(const float* qkv, int64_t ld, const float* kc, const float*
     AttnRowsParams p{qkv, ld, kc, vc, seq_stride, posv, seqv, att, ld_att, part, counters, H, HKV, nsplit, per, scale};
     const dim3 grid{unsigned(B), unsigned(HKV), unsigned(nsplit)};
     const int group = H / HKV;
-    if (group <= 2) k_attn_rows<2><<<grid, AR_THREADS, 0, s>>>(p);
-    else if (group <= 4) k_attn_rows<4><<<grid, AR_THREADS, 0, s>>>(p);
-    else k_attn_rows<8><<<grid, AR_THREADS, 0, s>>>(p);
-    ELB_CUDA(cudaGetLastError());
-    return ELB_OK;
+    return launch_after(group <= 2 ? k_attn_rows<2> : group <= 4 ? k_attn_rows<4> : k_attn_rows<8>, grid, dim3(AR_THREADS), 0, s, pdl, p);
 }
 
 // ---------------------------------------------------------------- RMSNorm over rows (el::rmsnorm, src/ops.cpp:155-160)
@@ -849,11 +848,9 @@ int attn_decode_launch(const AttnDecodeArgs& a, cudaStream_t s) {
 
 int qkv_post_launch(float* qkv, int64_t ld, const float* q_norm, const float* k_norm, const float* rope, int pos0, int B,
                     float* kc, float* vc, int H, int HKV, int rope_dim, float eps, cudaStream_t s, const int* posv,
-                    const int* seqv, size_t seq_stride) {
-    k_qkv_post<<<dim3(B, (H + 2 * HKV + 7) / 8), dim3(32, 8), 0, s>>>(qkv, ld, q_norm, k_norm, reinterpret_cast<const float2*>(rope), pos0, kc,
-                                                   vc, H, HKV, rope_dim, eps, posv, seqv, seq_stride);
-    ELB_CUDA(cudaGetLastError());
-    return ELB_OK;
+                    const int* seqv, size_t seq_stride, bool pdl) {
+    return launch_after(k_qkv_post, dim3(B, (H + 2 * HKV + 7) / 8), dim3(32, 8), 0, s, pdl, qkv, ld, q_norm, k_norm,
+                        reinterpret_cast<const float2*>(rope), pos0, kc, vc, H, HKV, rope_dim, eps, posv, seqv, seq_stride);
 }
 
 size_t attn_prefill_scratch_floats(int max_batch, int H, int HKV) {  // partial results of the chunked prompt attention

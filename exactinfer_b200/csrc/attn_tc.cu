@@ -74,6 +74,8 @@ __global__ void __launch_bounds__(256) k_kv_split16(const float* __restrict__ kc
                                                     __half* __restrict__ kh, __half* __restrict__ kl, __half* __restrict__ vth,
                                                     __half* __restrict__ vtl) {
     __shared__ float vs[32][65];
+    pdl_launch_dependents();
+    pdl_wait();
     const int t0 = blockIdx.x * 32, d0 = blockIdx.y * 64, tid = threadIdx.x;
     for (int i = tid; i < 32 * 32; i += 256) {  // keys: 32 x 32 pairs of dimensions
         const int j = i >> 5, c = (i & 31) * 2;
@@ -123,6 +125,7 @@ __global__ void __launch_bounds__(AT_THREADS, 2) k_attn_prefill_tc(const AtParam
     __shared__ int s_last;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int kvh = blockIdx.x, group = p.H / p.HKV, TQ = AT_ROWS / group, n_qt = (p.B + TQ - 1) / TQ;
+    pdl_wait();
     // item -> (query tile, chunk), the last query tiles first: theirs are the full chunks, and a short one fits behind them
     int qt = n_qt - 1, chunk = int(blockIdx.y), n_chunks = at_chunks(p.pos0, p.B, TQ, qt, p.kchunk);
     while (chunk >= n_chunks && qt > 0) {
@@ -377,7 +380,7 @@ bool attn_prefill_tc_usable(int H, int HKV, int64_t ld, int64_t ld_att) {
 // part / counters: the scratch of attn_prefill_launch (same sizes); kv16: attn_prefill_tc_scratch_halves(n_ctx, HKV * 128) halves
 int attn_prefill_tc_launch(const float* qkv, int64_t ld, const float* kc, const float* vc, float* att, int64_t ld_att, int pos0,
                            int B, int H, int HKV, float scale, cudaStream_t s, float* part, unsigned* counters, void* kv16, int max_batch,
-                           int sm_count) {
+                           int sm_count, bool pdl) {
     if (!attn_prefill_tc_usable(H, HKV, ld, ld_att) || !kv16 || !part || !counters)
         return fail(ELB_ERR_STATE, "attention: tensor-core prompt attention not usable here");
     const int T = pos0 + B, Tp = (T + AT_K - 1) / AT_K * AT_K, KD = HKV * D, group = H / HKV, TQ = AT_ROWS / group;
@@ -385,8 +388,7 @@ int attn_prefill_tc_launch(const float* qkv, int64_t ld, const float* kc, const 
     __half* kl = kh + size_t(Tp) * KD;
     __half* vth = kl + size_t(Tp) * KD;
     __half* vtl = vth + size_t(Tp) * KD;
-    k_kv_split16<<<dim3(Tp / 32, KD / 64), 256, 0, s>>>(kc, vc, T, Tp, KD, kh, kl, vth, vtl);
-    ELB_CUDA(cudaGetLastError());
+    ELB_TRY(launch_after(k_kv_split16, dim3(Tp / 32, KD / 64), dim3(256), 0, s, pdl, kc, vc, T, Tp, KD, kh, kl, vth, vtl));
     ELB_TRY(ensure_dyn_smem(reinterpret_cast<const void*>(k_attn_prefill_tc), AT_SMEM));
     const int n_qt = (B + TQ - 1) / TQ, tiles_max = Tp / AT_K;
     // How many tiles of 64 keys a CTA walks, from what the launch would then take, in tile times (6 us with one CTA on an SM;
@@ -411,9 +413,7 @@ int attn_prefill_tc_launch(const float* qkv, int64_t ld, const float* kc, const 
         if (cut == 1 || cost < best) { best = cost; kchunk = k; items = n; }
     }
     AtParams p{qkv, ld, kh, kl, vth, vtl, Tp, KD, att, ld_att, pos0, B, H, HKV, kchunk, (tiles_max + kchunk - 1) / kchunk, scale, part, counters};
-    k_attn_prefill_tc<<<dim3(HKV, items), AT_THREADS, AT_SMEM, s>>>(p);
-    ELB_CUDA(cudaGetLastError());
-    return ELB_OK;
+    return launch_after(k_attn_prefill_tc, dim3(HKV, items), dim3(AT_THREADS), AT_SMEM, s, pdl, p);
 }
 
 }  // namespace elb

@@ -176,6 +176,26 @@ __device__ __forceinline__ Pow2 make_pow2(int k) {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Launch behind the stream's previous kernel; pdl: the kernel starts while that one ends. It must then wait (pdl_wait, every
+// thread) before it touches memory, and a kernel that lets its successor go early has all its CTAs started by then. With it
+// on the attention kernels too, a 77-token turn of the 0.6B shape 3.03 -> 2.90 ms, a step of 16 rows of the 4B shape
+// 4.60 -> 4.44, of 64 rows of the 1.7B shape 5.32 -> 5.18.
+template <class... P, class... A>
+inline int launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    ELB_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    return ELB_OK;
+}
+
 // ---------------------------------------------------------------- host-side declarations shared between files
 struct DeviceInfo {
     int sm_count = 0;
@@ -265,13 +285,13 @@ struct AttnDecodeArgs {
 int attn_decode_launch(const AttnDecodeArgs& a, cudaStream_t s);
 int qkv_post_launch(float* qkv, int64_t ld, const float* q_norm, const float* k_norm, const float* rope, int pos0, int B,
                     float* kc, float* vc, int H, int HKV, int rope_dim, float eps, cudaStream_t s,
-                    const int* posv = nullptr, const int* seqv = nullptr, size_t seq_stride = 0);
+                    const int* posv, const int* seqv, size_t seq_stride, bool pdl);
 // rows of several sequences (row b: position posv[b] of sequence seqv[b]; posv_host: the positions on the host); part:
 // attn_rows_part_floats(H) floats, counters [B][HKV] zero at first
 size_t attn_rows_part_floats(int H);
 int attn_rows_launch(const float* qkv, int64_t ld, const float* kc, const float* vc, size_t seq_stride, const int* posv,
                      const int* seqv, const int* posv_host, float* att, int64_t ld_att, float* part, unsigned* counters, int B, int H,
-                     int HKV, float scale, int sm_count, cudaStream_t s);
+                     int HKV, float scale, int sm_count, cudaStream_t s, bool pdl);
 int attn_prefill_launch(const float* qkv, int64_t ld, const float* kc, const float* vc, float* att, int64_t ld_att,
                         int pos0, int B, int H, int HKV, float scale, cudaStream_t s, float* part = nullptr,
                         unsigned* counters = nullptr);
@@ -280,7 +300,7 @@ bool attn_prefill_tc_usable(int H, int HKV, int64_t ld, int64_t ld_att);
 size_t attn_prefill_tc_scratch_halves(int n_ctx, int KD);
 int attn_prefill_tc_launch(const float* qkv, int64_t ld, const float* kc, const float* vc, float* att, int64_t ld_att, int pos0,
                            int B, int H, int HKV, float scale, cudaStream_t s, float* part, unsigned* counters, void* kv16, int max_batch,
-                           int sm_count);
+                           int sm_count, bool pdl);
 size_t attn_prefill_scratch_floats(int max_batch, int H, int HKV);  // `part` of attn_prefill_launch
 size_t attn_prefill_counters(int max_batch, int H, int HKV);        // `counters` (zero before the first launch)
 int rmsnorm_launch(float* out, const float* x, const float* w, int n, float eps, int rows, cudaStream_t s);

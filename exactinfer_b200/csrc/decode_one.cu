@@ -22,6 +22,9 @@
 //     unit ranges: a row tile then has at most two contributing CTAs, whose sums the next conversion adds;
 //   * an ffn_down activation too long for shared memory (25 600 values of the 32B shape: 121 KB of limbs) is worked
 //     off in down_parts equal ranges of k: convert one, multiply it, convert the next.
+//     The words are relaxed: what separates the emptying of a word from its next reader is a whole layer, five exchanges
+//     that every CTA takes part in (tens of microseconds). A fence per stage on every thread was measured and costs 17 % of
+//     a step of the 0.6B shape, 7 % of the 4B shape, 1.6 % of the 32B shape.
 // All waits are bounded: on timeout the kernel raises an error word, drains its copies and leaves.
 #include <cuda.h>
 

@@ -239,14 +239,14 @@ int body_prefill(Model* m, int B, int pos0, int seq0 = 0, const int* posv_host =
         for (auto& s : L.qkv) ELB_TRY(linear_tokens(m, s.w, m->x, E, L.attn_norm, B, m->qkv + s.col, QKV, nullptr, EPI_STORE, m->nl_qkv));
         if (mixed) {
             ELB_TRY(qkv_post_launch(m->qkv, QKV, L.q_norm, L.k_norm, m->rope, 0, B, kc, vc, H, HKV, c.rope_dim, c.eps, m->stream,
-                                    m->posv_dev, m->seq_dev, seq_stride));
+                                    m->posv_dev, m->seq_dev, seq_stride, m->use_pdl));
             ELB_TRY(attn_rows_launch(m->qkv, QKV, kc, vc, seq_stride, m->posv_dev, m->seq_dev, posv_host, m->att, QD,
-                                     m->rows_part, m->rows_counters, B, H, HKV, scale, m->sm_count, m->stream));
+                                     m->rows_part, m->rows_counters, B, H, HKV, scale, m->sm_count, m->stream, m->use_pdl));
         } else {
-            ELB_TRY(qkv_post_launch(m->qkv, QKV, L.q_norm, L.k_norm, m->rope, pos0, B, kc, vc, H, HKV, c.rope_dim, c.eps, m->stream));
+            ELB_TRY(qkv_post_launch(m->qkv, QKV, L.q_norm, L.k_norm, m->rope, pos0, B, kc, vc, H, HKV, c.rope_dim, c.eps, m->stream, nullptr, nullptr, 0, m->use_pdl));
             if (m->kv16 && attn_prefill_tc_usable(H, HKV, QKV, QD)) {
                 ELB_TRY(attn_prefill_tc_launch(m->qkv, QKV, kc, vc, m->att, QD, pos0, B, H, HKV, scale, m->stream, m->ap_part, m->ap_counters, m->kv16,
-                                               m->max_batch, m->sm_count));
+                                               m->max_batch, m->sm_count, m->use_pdl));
                 ++m->launches;  // the fp16 split of the layer's keys and values
             } else {
                 ELB_TRY(attn_prefill_launch(m->qkv, QKV, kc, vc, m->att, QD, pos0, B, H, HKV, scale, m->stream, m->ap_part, m->ap_counters));
