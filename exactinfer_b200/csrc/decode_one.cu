@@ -137,7 +137,8 @@ __device__ __forceinline__ void d1_tensor_copy(uint32_t dst, const void* map, in
 
 // Prefetch cursor: the next unit of a warp's stream that has not been requested yet.
 struct Cursor1 {
-    int l, i, left, b, upt, ub, skip, tile;  // left: units of this range; b: k block within the row tile
+    int l, i, left, b, upt, ub, skip, tile;  // left: units of this range; b: k block within the row tile's part
+    int k0;                                  // F16: k block at which the part starts (quantized: src is there already)
     const uint8_t* src;                      // the unit (F16: the matrix's tensor map)
 };
 __device__ __forceinline__ void d1_seek(const DkParams& p, Cursor1& c, const Share* shares) {  // first non-empty range from (l, i) on
@@ -153,11 +154,13 @@ __device__ __forceinline__ void d1_seek(const DkParams& p, Cursor1& c, const Sha
             c.ub = d1_unit_bytes(type);
             const uint8_t* W = p.W[c.l][wi];
             c.tile = sh.tile;
+            const int part0 = kind >= K1_DOWN ? (kind - K1_DOWN) * c.upt : 0;  // first unit of the part within a row tile
             if (type == ELB_F16) {
+                c.k0 = part0;
                 c.src = p.f16_maps + size_t(c.l * DK_LAYER_MATS + wi) * 128;
             } else {
                 c.skip = (full.upt - c.upt) * c.ub;
-                c.src = W + (size_t(sh.tile) * full.upt + (kind >= K1_DOWN ? (kind - K1_DOWN) * c.upt : 0) + c.b) * c.ub;
+                c.src = W + (size_t(sh.tile) * full.upt + part0 + c.b) * c.ub;
             }
             return;
         }
@@ -191,7 +194,7 @@ __device__ __noinline__ void d1_producer(const DkParams& p, const uint32_t ring0
                 const uint32_t bar = bars + (seq % DK_NBAR) * 8u, dst = base + uint32_t(off);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(ub) : "memory");
                 if (F16M) {
-                    d1_tensor_copy(dst, c.src, c.b * 128, c.tile * 16, bar);
+                    d1_tensor_copy(dst, c.src, (c.k0 + c.b) * 128, c.tile * 16, bar);
                 } else {
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                                  ::"r"(dst), "l"(c.src), "r"(ub), "r"(bar)

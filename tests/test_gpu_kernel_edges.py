@@ -105,9 +105,11 @@ def test_decode_across_attention_splits(elb, layout, heads, kv):
     assert decode_pair(elb, spec, 31, 700, (0, 59, 60, 61, 650, 3, 651, 120)) <= 2e-4
 
 
-# a feed-forward vector whose limbs do not fit in shared memory beside the weight rings: worked off in parts along k
-def test_decode_long_feed_forward(elb):
-    spec = synth.Spec(name="small", n_layer=2, n_embd=256, n_ff=25600, n_head=2, n_head_kv=1, n_vocab=640, layout="q4_k_m",
+# a feed-forward vector whose limbs (or fp32 values: F16) do not fit in shared memory beside the weight rings: worked off
+# in two and in four parts along k, which every weight format walks with coordinates of its own
+@pytest.mark.parametrize("layout,n_ff", (("q4_k_m", 25600), ("f16", 25600), ("q8_0", 25600), ("q6_k", 25600), ("f16", 57344), ("q4_k_m", 57344)))
+def test_decode_long_feed_forward(elb, layout, n_ff):
+    spec = synth.Spec(name="small", n_layer=2, n_embd=256, n_ff=n_ff, n_head=2, n_head_kv=1, n_vocab=640, layout=layout,
                       head_sigma=2e-5)
     assert decode_pair(elb, spec, 32, 80, (0, 17, 70)) <= 2e-4
 
