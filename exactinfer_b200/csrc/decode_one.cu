@@ -628,11 +628,11 @@ __device__ __forceinline__ void d1_attention(const DkParams& p, const int l, con
             ex_put(att, size_t(QD), par, size_t(kvh * group) * DK_HD + f0 * 4 + e, o / L);
         }
     }
-    // Slots of splits that this step does not have may hold words of an earlier step with more keys: emptied in the first
-    // two layers (one half each), before a longer step could take them for its own.
+    // Slots that this step does not write may hold words of an earlier step with more keys (one split writes none at all, not
+    // even slot 0): emptied in the first two layers (one half each), before a longer step could take them for its own.
     if (l < 2)
 #pragma unroll 1
-        for (int q = split + ns; q < p.nsplit; q += ns)
+        for (int q = ns == 1 ? 0 : split + ns; q < p.nsplit; q += ns)
 #pragma unroll 1
             for (int i = threadIdx.x; i < pstride; i += D1_WORKERS) ex_st(part + size_t(par ^ 1) * psize + size_t(q) * pstride + i, D1_EMPTY);
     d1_sync();  // the scratch area is the next conversion's

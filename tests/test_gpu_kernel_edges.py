@@ -96,13 +96,37 @@ def decode_pair(elb, spec, seed, n_ctx, walk):
     return worst
 
 
-# attention splits of 60 keys: one, two, many, back to one, many again (stale partial results must not be taken); every
-# group size of query heads the kernel is compiled for; all-F16 and quantized weights; an odd number of layers
+# attention splits of 60 keys: one, two, many, back to one, many again; every group size of query heads the kernel is
+# compiled for; all-F16 and quantized weights; an odd number of layers
 @pytest.mark.parametrize("layout,heads,kv", (("q4_k_m", 8, 4), ("f16", 6, 2), ("q8_0", 8, 1), ("q6_k", 2, 2)))
 def test_decode_across_attention_splits(elb, layout, heads, kv):
     spec = synth.Spec(name="small", n_layer=3, n_embd=512, n_ff=768, n_head=heads, n_head_kv=kv, n_vocab=1111, layout=layout,
                       head_sigma=2e-5)
     assert decode_pair(elb, spec, 31, 700, (0, 59, 60, 61, 650, 3, 651, 120)) <= 2e-4
+
+
+# single evaluations at long and short contexts in turn, with an odd and an even number of short ones in between: what a step
+# with several key splits leaves in the exchange buffers must not be taken for a later step's, whatever the number of layers
+@pytest.mark.parametrize("n_layer", (1, 2, 3, 5))
+def test_decode_long_and_short_contexts_in_turn(elb, n_layer):
+    spec = synth.Spec(name="small", n_layer=n_layer, n_embd=512, n_ff=768, n_head=8, n_head_kv=2, n_vocab=640, layout="q8_0",
+                      head_sigma=2e-5)
+    tens = list(synth.generate(spec, 41))
+    gpu, cpu = elb.Backend(spec, tens, 704), ol.OracleModel(spec, tens, 704)
+    toks = synth.lcg_tokens(704, spec.n_vocab, 41)
+    gpu.eval(toks[:700], 0, want_logits=False)
+    cpu.eval(toks[:700], 0)
+    walk = (650, 5, 651, 7, 8, 9, 100, 5, 699, 5, 6, 650, 59, 60, 59, 61, 58, 400)
+    seen = {}
+    for pos in sorted(set(walk)):  # (upwards first: a row of the cache then is what a single step writes, and stays so)
+        seen[pos], want = gpu.eval(toks[pos:pos + 1], pos), cpu.eval(toks[pos:pos + 1], pos)
+        assert gpu.last_eval_stats()[1] == 1, "the persistent kernel must run"
+        assert np.abs(seen[pos] - want).max() <= 2e-4 * np.abs(want).max(), pos
+    for _ in range(60):
+        for pos in walk:
+            assert np.array_equal(gpu.eval(toks[pos:pos + 1], pos), seen[pos]), pos
+    gpu.close()
+    cpu.close()
 
 
 # a feed-forward vector whose limbs (or fp32 values: F16) do not fit in shared memory beside the weight rings: worked off
