@@ -15,6 +15,9 @@ constexpr int DK_LAYER_MATS = 6;   // matrices of a layer in execution order: n_
 constexpr int DK_MAX_PARTS = 4;     // most parts ffn_down is cut into along k (decode_one.cu)
 constexpr int DK_ONE_KINDS = 6 + DK_MAX_PARTS;
 
+// Exchange word of decode_one.cu: a value and the number of the layer pass it belongs to, loaded and stored as one
+struct alignas(8) DkEx { float v; unsigned num; };
+
 struct DkKind {  // one kind of weight matrix, in tiled layout
     int tiles, upt, rows, n;
     // How the CTAs share the matrix. group_tiles / group_off: the matrix is tiles [group_off, group_off + tiles) of a
@@ -75,10 +78,10 @@ struct DkParams {
     int slots;              // row-tile slots per warp in the reduction buffer
     int cta_tiles;          // most row tiles a CTA's share of a matrix can touch
     int n_max;              // longest activation vector
-    // decode_one.cu: the vectors that pass between CTAs, each twice (one half per layer, in turn)
-    float *ex_e, *ex_q, *ex_a, *ex_p1, *ex_g, *ex_p2, *ex_s;  // embedding row, q|k|v, att, partial sums [2][E], act, partial sums, attention splits
+    // decode_one.cu: the vectors that pass between CTAs
+    DkEx *ex_e, *ex_q, *ex_a, *ex_p1, *ex_g, *ex_p2, *ex_s;  // embedding row, q|k|v, att, partial sums [2][E], act, partial sums [2][E], attention splits
     unsigned* fin;          // CTAs that have finished the step (zero between launches)
-    int qkv_len;            // floats of q|k|v
+    int qkv_len;            // values of q|k|v
     const uint8_t* f16_maps;  // F16: tensor maps of the matrices [n_layer + 1][DK_LAYER_MATS]
     int f16;                // every matrix is F16 (otherwise every one is quantized)
     int down_parts;         // equal ranges of k in which ffn_down is worked off
@@ -92,7 +95,8 @@ struct DkParams {
 };
 
 // decode_one.cu (one GPU)
-size_t decode_one_exchange(DkParams& p, float* base);
+size_t decode_one_exchange(DkParams& p, uint8_t* base);
+int64_t decode_one_steps(const DkParams& p);
 int decode_one_ring_bytes(const DkParams& p, int max_unit, int min_unit, int device);
 int decode_one_fits(const DkParams& p, int ring_bytes, int device, bool* fits);
 int decode_one_launch(const DkParams& p, int ring_bytes, int grid, cudaStream_t s);

@@ -3,15 +3,17 @@
 // At batch 1 every layer is a chain of five dependent steps (q|k|v, attention, output projection, gate|up, down), each a
 // few microseconds of HBM traffic: what bounds the step is the latency of handing a vector of a few thousand values from
 // every SM to every SM, five times per layer. Here one CTA per SM stays resident for the whole step and
-//   * a value IS its own arrival flag: the vectors that pass between CTAs lie in exchange buffers whose words hold a
-//     pattern that no result has (D1_EMPTY) until they are written; a consumer loads its words and asks again for those
-//     that are still empty. There is no barrier, no fence and no counter between a producer's store and a consumer's
-//     load, and a block of the activation is converted as soon as its own words are there. Every buffer exists twice;
-//     layer n uses half n & 1, and whoever writes a word of one half empties the same word of the other, whose readers
-//     are done by then: the writer of exchange s of layer n + 1 has consumed exchange s - 1 of that layer in full, hence
-//     (going back one exchange at a time) exchange s + 1 of layer n, which its producers wrote after they had read all
-//     of exchange s of layer n (CTAs without a share in a stage: see d1_keep_rows). With the grid barriers of decode.cu (release, poll, then load: 2.5 us from the last
-//     store to the first use, against about 1 us) the 4B-shape layer took 48.7 us, here 35.2 us;
+//   * a value travels with the number of the layer pass it belongs to, in ONE 8-byte word written by one store: a consumer
+//     loads its words and asks again for those that do not carry the number it waits for. There is no barrier, no fence and
+//     no counter between a producer's store and a consumer's load, a word of another layer or step is never taken for this
+//     one's, whatever the order in which stores arrive, and a block of the activation is converted as soon as its own words
+//     are there. One buffer per vector is enough: whoever reads exchange s of layer n afterwards writes something that,
+//     going from exchange to exchange, every writer of exchange s of layer n + 1 has waited for (a CTA reads nothing in a
+//     stage in which it has no share, except the rows of the residual stream that its next share adds to). With the grid
+//     barriers of decode.cu (release, poll, then load: 2.5 us from the last store to the first use, against about 1 us) the
+//     4B-shape layer took 48.7 us, here 35.5 us. (Partial sums in 16-byte words of three values and the number, a quarter
+//     fewer bytes: a step 2 % slower on the 0.6B and 1.7B shapes, 1 % faster on the 4B and 32B shapes. All vectors so: 5 %
+//     slower on the 0.6B and 4B shapes; two producers then share a 32-byte sector of the feed-forward vector.);
 //   * every working warp owns a fixed, contiguous share of the (row tile, k block) units of every weight matrix of the
 //     step, in execution order, and a producer warp keeps every working warp's ring in shared memory as full as it gets,
 //     no matter what the CTA is doing: HBM streams through exchanges, attention and conversion;
@@ -22,9 +24,6 @@
 //     unit ranges: a row tile then has at most two contributing CTAs, whose sums the next conversion adds;
 //   * an ffn_down activation too long for shared memory (25 600 values of the 32B shape: 121 KB of limbs) is worked
 //     off in down_parts equal ranges of k: convert one, multiply it, convert the next.
-//     The words are relaxed: what separates the emptying of a word from its next reader is a whole layer, five exchanges
-//     that every CTA takes part in (tens of microseconds). A fence per stage on every thread was measured and costs 17 % of
-//     a step of the 0.6B shape, 7 % of the 4B shape, 1.6 % of the 32B shape.
 // All waits are bounded: on timeout the kernel raises an error word, drains its copies and leaves.
 #include <cuda.h>
 
@@ -44,7 +43,6 @@ namespace {
 constexpr int D1_WARPS = 15, D1_WORKERS = 32 * D1_WARPS, D1_THREADS = D1_WORKERS + 32;
 static_assert(D1_WARPS <= DK_WARPS, "the ring bookkeeping has one place per warp");
 __device__ __forceinline__ void d1_sync() { asm volatile("bar.sync 1, %0;" ::"n"(D1_WORKERS) : "memory"); }
-constexpr uint32_t D1_EMPTY = 0xFFFFFFFFu;      // a NaN with a payload that no operation produces
 constexpr unsigned D1_POLL_LIMIT = 1u << 20;    // loads of one wait for an exchange word: about a second
 constexpr int D1_SPLIT_KEYS = 4 * D1_WARPS;     // keys of one attention split: one tile of 4 keys per warp
 constexpr int D1_F16_UNIT = 16 * 128 * 2;       // F16: 16 rows x 128 k
@@ -64,25 +62,38 @@ __device__ __forceinline__ bool d1_sync_dead(const int* dead) {
 
 // ---------------------------------------------------------------- exchange words
 
-__device__ __forceinline__ float4 ex_ld4(const float* p) {
-    float4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
-    return v;
+// A word is one memory location: loads and stores are relaxed, at GPU scope, 64 bits each.
+__device__ __forceinline__ DkEx ex_word(unsigned long long w) { return DkEx{__uint_as_float(unsigned(w)), unsigned(w >> 32)}; }
+__device__ __forceinline__ DkEx ex_ld(const DkEx* p) {
+    unsigned long long a;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
+    return ex_word(a);
 }
-__device__ __forceinline__ float ex_ld(const float* p) {
-    float v;
-    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
-    return v;
+__device__ __forceinline__ void ex_ld2(const DkEx* p, DkEx& x, DkEx& y) {  // two words (p: 16-byte aligned)
+    unsigned long long a, b;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+    x = ex_word(a);
+    y = ex_word(b);
 }
-__device__ __forceinline__ void ex_st(float* p, uint32_t bits) { asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(bits) : "memory"); }
-__device__ __forceinline__ bool ex_empty(float v) { return __float_as_uint(v) == D1_EMPTY; }
-__device__ __forceinline__ bool ex_empty(const float4& v) { return ex_empty(v.x) || ex_empty(v.y) || ex_empty(v.z) || ex_empty(v.w); }
-// word i of the half `par` of a buffer (halves of `size` floats); the same word of the other half becomes empty
-__device__ __forceinline__ void ex_put(float* buf, size_t size, int par, size_t i, float v) {
-    const uint32_t b = __float_as_uint(v);
-    ex_st(buf + size_t(par ^ 1) * size + i, D1_EMPTY);
-    ex_st(buf + size_t(par) * size + i, b == D1_EMPTY ? 0x7FFFFFFFu : b);
+__device__ __forceinline__ void ex_st(DkEx* p, float v, unsigned num) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((unsigned long long)num << 32 | __float_as_uint(v)) : "memory");
 }
+struct Ex8 {  // eight consecutive words (64-byte aligned)
+    unsigned long long w[8];
+    __device__ __forceinline__ void load(const DkEx* p) {
+#pragma unroll
+        for (int j = 0; j < 8; j += 4)
+            asm volatile("ld.relaxed.gpu.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                         : "=l"(w[j]), "=l"(w[j + 1]), "=l"(w[j + 2]), "=l"(w[j + 3]) : "l"(p + j) : "memory");
+    }
+    __device__ __forceinline__ bool missing(unsigned num) const {
+        bool m = false;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) m = m || unsigned(w[j] >> 32) != num;
+        return m;
+    }
+    __device__ __forceinline__ float4 get(int j) const { return make_float4(ex_word(w[j]).v, ex_word(w[j + 1]).v, ex_word(w[j + 2]).v, ex_word(w[j + 3]).v); }
+};
 struct Wait {  // of one place where a thread waits for words; false: give up (a wait has run out here or elsewhere in the CTA)
     unsigned it = 0;
     __device__ __forceinline__ bool again(const DkParams& p, int* dead) {
@@ -245,40 +256,45 @@ struct Rows {
 // limbs, or fp32 values (F16M). NORM multiplies by norm_w; the factor 1 / sqrt(mean(x^2) + eps) of the RMSNorm
 // (src/ops.cpp:155-160 of the reference, sum of squares in double) is applied to the row sums of the matvec, and every
 // warp leaves its share of the sum of squares in red8: no block waits for the sum over the vector. Warp w takes blocks
-// w, w + 15, ...; the words of the next blocks are asked for before the current one is converted (a loop, not unrolled:
-// the code of a conversion runs once or twice per stage, as fast as it can be fetched).
+// w, w + 15, ...; the words of the next block (plain: of the two next) are asked for before the current one is converted,
+// into the registers of the words just used (a loop, not unrolled: the code of a conversion runs once or twice per stage, as
+// fast as it can be fetched).
 template <bool NORM, bool F16M>
-__device__ __forceinline__ void d1_convert(const DkParams& p, const float* A, const float* B, const float* norm_w, const int blk0,
-                                           const int nblk, const int nl, const ActSmem& a, const int sd_mask, double* red8, const Rows& rows,
-                                           int* dead) {
+__device__ __forceinline__ void d1_convert(const DkParams& p, const DkEx* A, const DkEx* B, const unsigned num, const float* norm_w,
+                                           const int blk0, const int nblk, const int nl, const ActSmem& a, const int sd_mask, double* red8,
+                                           const Rows& rows, int* dead) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    A += size_t(blk0) * 256 + lane * 8;
+    A += blk0 * 256 + lane * 8;
     if (NORM) { norm_w += lane * 8; if (B) B += lane * 8; }
     double ss = 0.0;
-    float4 v0 = z, v1 = z, w0 = z, w1 = z;      // the current block's words
-    float4 x0 = z, x1 = z, y0 = z, y1 = z;      // the next block's (plain: and the one behind it)
+    Ex8 va{}, vb{};   // the current block's words (plain: vb, the next block's)
     if (warp < nblk) {
-        v0 = ex_ld4(A + warp * 256); v1 = ex_ld4(A + warp * 256 + 4);
-        if (NORM && B) { w0 = ex_ld4(B + warp * 256); w1 = ex_ld4(B + warp * 256 + 4); }
+        va.load(A + warp * 256);
+        if (NORM && B) vb.load(B + warp * 256);
     }
-    if (warp + D1_WARPS < nblk) { x0 = ex_ld4(A + (warp + D1_WARPS) * 256); x1 = ex_ld4(A + (warp + D1_WARPS) * 256 + 4); }
-    if (!NORM && warp + 2 * D1_WARPS < nblk) { y0 = ex_ld4(A + (warp + 2 * D1_WARPS) * 256); y1 = ex_ld4(A + (warp + 2 * D1_WARPS) * 256 + 4); }
+    if (!NORM && warp + D1_WARPS < nblk) vb.load(A + (warp + D1_WARPS) * 256);
 #pragma unroll 1
     for (int b = warp; b < nblk; b += D1_WARPS) {
         const int at = b * 256;
-        float4 n0 = z, n1 = z;
+        float4 n0, n1;
         if (NORM) { n0 = __ldg(reinterpret_cast<const float4*>(norm_w + at)); n1 = __ldg(reinterpret_cast<const float4*>(norm_w + at + 4)); }
         Wait wait;
-        while (__any_sync(0xffffffffu, ex_empty(v0) || ex_empty(v1) || (NORM && (ex_empty(w0) || ex_empty(w1))))) {
-            v0 = ex_ld4(A + at); v1 = ex_ld4(A + at + 4);
-            if (NORM && B) { w0 = ex_ld4(B + at); w1 = ex_ld4(B + at + 4); }
+        while (__any_sync(0xffffffffu, va.missing(num) || (NORM && B && vb.missing(num)))) {
+            va.load(A + b * 256);
+            if (NORM && B) vb.load(B + b * 256);
             if (__any_sync(0xffffffffu, !wait.again(p, dead))) break;
         }
+        float4 v0 = va.get(0), v1 = va.get(4);
+        const int next = b + D1_WARPS;
         if (NORM) {
             if (B) {
+                const float4 w0 = vb.get(0), w1 = vb.get(4);
                 v0 = make_float4(__fadd_rn(v0.x, w0.x), __fadd_rn(v0.y, w0.y), __fadd_rn(v0.z, w0.z), __fadd_rn(v0.w, w0.w));
                 v1 = make_float4(__fadd_rn(v1.x, w1.x), __fadd_rn(v1.y, w1.y), __fadd_rn(v1.z, w1.z), __fadd_rn(v1.w, w1.w));
+            }
+            if (next < nblk) {
+                va.load(A + next * 256);
+                if (B) vb.load(B + next * 256);
             }
             ss += double(v0.x) * v0.x + double(v0.y) * v0.y + double(v0.z) * v0.z + double(v0.w) * v0.w;
             ss += double(v1.x) * v1.x + double(v1.y) * v1.y + double(v1.z) * v1.z + double(v1.w) * v1.w;
@@ -293,6 +309,9 @@ __device__ __forceinline__ void d1_convert(const DkParams& p, const float* A, co
             }
             v0 = make_float4(__fmul_rn(v0.x, n0.x), __fmul_rn(v0.y, n0.y), __fmul_rn(v0.z, n0.z), __fmul_rn(v0.w, n0.w));
             v1 = make_float4(__fmul_rn(v1.x, n1.x), __fmul_rn(v1.y, n1.y), __fmul_rn(v1.z, n1.z), __fmul_rn(v1.w, n1.w));
+        } else {
+            va = vb;
+            if (next + D1_WARPS < nblk) vb.load(A + (next + D1_WARPS) * 256);
         }
         if (F16M) {
             float* dst = reinterpret_cast<float*>(a.lim) + at + lane * 8;
@@ -301,16 +320,6 @@ __device__ __forceinline__ void d1_convert(const DkParams& p, const float* A, co
         } else {
             split_block(v0, v1, b, nl, a, sd_mask, lane);
         }
-        v0 = x0; v1 = x1;
-        if (NORM) {
-            const int nx = b + D1_WARPS, ny = nx + D1_WARPS;
-            if (B && nx < nblk) { w0 = ex_ld4(B + nx * 256); w1 = ex_ld4(B + nx * 256 + 4); }
-            if (ny < nblk) { x0 = ex_ld4(A + ny * 256); x1 = ex_ld4(A + ny * 256 + 4); }
-        } else {
-            const int ny = b + 3 * D1_WARPS;
-            x0 = y0; x1 = y1;
-            if (ny < nblk) { y0 = ex_ld4(A + ny * 256); y1 = ex_ld4(A + ny * 256 + 4); }
-        }
     }
     if (NORM) {
         ss = warp_sum(ss);
@@ -318,30 +327,31 @@ __device__ __forceinline__ void d1_convert(const DkParams& p, const float* A, co
     }
 }
 
-// A CTA without a share in the matrices of a stage still needs its rows of the residual stream. all: it also waits for
-// every word. A CTA must not come to a stage of layer n before all exchanges of layer n - 1 are complete (the half it
-// would read still holds layer n - 2's words until then): a CTA with shares learns that from what it consumes, the others
-// wait for the whole stream once per layer.
-__device__ __noinline__ void d1_keep_rows(const DkParams& p, const float* A, const float* B, const Rows rows, const bool all, int* dead) {
-    auto get = [&](int i) {
-        float4 a = ex_ld4(A + i), b = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (B) b = ex_ld4(B + i);
+// A CTA without a share in the matrices of a stage still needs its rows of the residual stream, and CTA b block b of the
+// last one.
+__device__ __noinline__ void d1_keep_rows(const DkParams& p, const DkEx* A, const DkEx* B, const unsigned num, const Rows rows, int* dead) {
+    auto get = [&](int i, float* dst) {
+        Ex8 a, b{};
+        a.load(A + i);
+        if (B) b.load(B + i);
         Wait wait;
-        while ((ex_empty(a) || ex_empty(b)) && wait.again(p, dead)) {
-            a = ex_ld4(A + i);
-            if (B) b = ex_ld4(B + i);
+        while ((a.missing(num) || (B && b.missing(num))) && wait.again(p, dead)) {
+            a.load(A + i);
+            if (B) b.load(B + i);
         }
-        if (!B) return a;
-        return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+        float4 v0 = a.get(0), v1 = a.get(4);
+        if (B) {
+            const float4 w0 = b.get(0), w1 = b.get(4);
+            v0 = make_float4(__fadd_rn(v0.x, w0.x), __fadd_rn(v0.y, w0.y), __fadd_rn(v0.z, w0.z), __fadd_rn(v0.w, w0.w));
+            v1 = make_float4(__fadd_rn(v1.x, w1.x), __fadd_rn(v1.y, w1.y), __fadd_rn(v1.z, w1.z), __fadd_rn(v1.w, w1.w));
+        }
+        *reinterpret_cast<float4*>(dst) = v0;
+        *reinterpret_cast<float4*>(dst + 4) = v1;
     };
 #pragma unroll 1
-    for (int i = (all ? 0 : rows.r0) + int(threadIdx.x) * 4; i < (all ? p.E : rows.r1); i += D1_WORKERS * 4) {
-        const float4 v = get(i);
-        if (i >= rows.r0 && i < rows.r1) *reinterpret_cast<float4*>(rows.keep + i - rows.r0) = v;
-    }
-    if (!rows.out) return;
-#pragma unroll 1
-    for (int i = blockIdx.x * 256 + int(threadIdx.x) * 4; i < p.E && threadIdx.x < 64; i = p.E) *reinterpret_cast<float4*>(rows.out + i) = get(i);
+    for (int i = rows.r0 + int(threadIdx.x) * 8; i < rows.r1; i += D1_WORKERS * 8) get(i, rows.keep + i - rows.r0);
+    const int o = blockIdx.x * 256 + int(threadIdx.x) * 8;
+    if (rows.out && threadIdx.x < 32 && o < p.E) get(o, rows.out + o);
 }
 
 // ---------------------------------------------------------------- matvec
@@ -353,7 +363,7 @@ struct Smem1 {
     float* red;    // [D1_WARPS][slots][16] row sums of each warp's share, per row tile it touches
     double* red8;  // [D1_WARPS]
     float* xrow;   // [2][row tiles of a share * 16]
-    int* flags;    // [2]: a wait has run out
+    int* flags;    // [2]: a wait has run out; [3]: the step's position
 };
 
 template <int TYPE>
@@ -454,7 +464,7 @@ __device__ __forceinline__ void d1_matvec(const DkParams& p, const int type, con
 //   0 q|k|v    -> exchange                        1, 3 attn_output, ffn_down: the CTA that holds a tile's first unit adds
 //   2 gate|up  -> silu(gate) * up -> exchange       the residual stream and writes vector 0, the one that holds its last
 //   4 head     -> logits                            unit vector 1 (a CTA that holds the whole tile: zeros)
-__device__ __forceinline__ void d1_epilogue(const DkParams& p, const int stage, const int kind, const int parts, const int seg, const int par,
+__device__ __forceinline__ void d1_epilogue(const DkParams& p, const int stage, const int kind, const int parts, const int seg, const unsigned num,
                                             const float inv, const Smem1& s, const float* xrow) {
     const int lane = threadIdx.x & 31;
     const CtaShare cs = s.cta[kind];
@@ -478,19 +488,18 @@ __device__ __forceinline__ void d1_epilogue(const DkParams& p, const int stage, 
         const int R = 16 * cs.tile + e;
         if (stage == 2) {  // rows 0..7 of a tile gate, 8..15 up (SwiGLU, src/model.cpp:222-225 of the reference)
             const float up = __shfl_down_sync(0xffffffffu, v, 8);
-            const int o = 8 * (cs.tile + lt) + row;
-            if (on && row < 8 && o < p.F) ex_put(p.ex_g, size_t(p.F), par, size_t(o), __fmul_rn(__fdiv_rn(v, 1.0f + expf(-v)), up));
+            if (on && row < 8) ex_st(p.ex_g + 8 * (cs.tile + lt) + row, __fmul_rn(__fdiv_rn(v, 1.0f + expf(-v)), up), num);
         } else if (on && R < rows) {
             if (stage == 0) {
-                ex_put(p.ex_q, size_t(p.qkv_len), par, size_t(p.qkv_col[seg] + R), v);
+                ex_st(p.ex_q + p.qkv_col[seg] + R, v, num);
             } else if (stage == 4) {
                 p.logits_peer[0][R] = v;
             } else {
-                float* buf = stage == 1 ? p.ex_p1 : p.ex_p2;
+                DkEx* buf = stage == 1 ? p.ex_p1 : p.ex_p2;
                 const bool first = lt > 0 || cs.first, last = lt + 1 < cs.tiles || cs.last;
                 if (first) v = __fadd_rn(xrow[e], v);
-                if (first && last) ex_put(buf, size_t(2) * p.E, par, size_t(p.E + R), 0.f);
-                ex_put(buf, size_t(2) * p.E, par, size_t((first ? 0 : p.E) + R), v);
+                if (first && last) ex_st(buf + p.E + R, 0.f, num);
+                ex_st(buf + (first ? 0 : p.E) + R, v, num);
             }
         }
     }
@@ -500,29 +509,30 @@ __device__ __forceinline__ void d1_epilogue(const DkParams& p, const int stage, 
 
 // RMSNorm over one 128-wide head followed by NEOX RoPE (src/ops.cpp:155-160, src/model.cpp:23-32 of the reference), as
 // dk_head_norm_rope, from exchange words; one warp per head, lane owns elements lane, lane+32, lane+64, lane+96.
-__device__ __forceinline__ void d1_head(const DkParams& p, const float* src, const float* w, const float2* cs, float* dst, int lane, int* dead) {
+__device__ __forceinline__ void d1_head(const DkParams& p, const DkEx* src, const unsigned num, const float* w, const float2* cs, float* dst, int lane, int* dead) {
     const int half = p.rope_dim / 2;
-    float v[4], wn[4];
+    DkEx x[4];
+    float wn[4];
     float2 c[2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = ex_ld(src + lane + 32 * j);
+    for (int j = 0; j < 4; ++j) x[j] = ex_ld(src + lane + 32 * j);
 #pragma unroll
     for (int j = 0; j < 4; ++j) wn[j] = __ldg(w + lane + 32 * j);
 #pragma unroll
     for (int j = 0; j < 2; ++j) c[j] = lane + 32 * j < half ? __ldg(cs + lane + 32 * j) : make_float2(1.f, 0.f);
     Wait wait;
-    while (__any_sync(0xffffffffu, ex_empty(v[0]) || ex_empty(v[1]) || ex_empty(v[2]) || ex_empty(v[3]))) {
+    while (__any_sync(0xffffffffu, x[0].num != num || x[1].num != num || x[2].num != num || x[3].num != num)) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = ex_ld(src + lane + 32 * j);
+        for (int j = 0; j < 4; ++j) x[j] = ex_ld(src + lane + 32 * j);
         if (__any_sync(0xffffffffu, !wait.again(p, dead))) break;
     }
     double ss = 0.0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) ss += double(v[j]) * v[j];
+    for (int j = 0; j < 4; ++j) ss += double(x[j].v) * x[j].v;
     ss = warp_sum(ss);
     const float inv = float(rsqrt_d(ss * (1.0 / DK_HD) + double(p.eps)));
 #pragma unroll
-    for (int j = 0; j < 4; ++j) dst[lane + 32 * j] = __fmul_rn(__fmul_rn(v[j], inv), wn[j]);
+    for (int j = 0; j < 4; ++j) dst[lane + 32 * j] = __fmul_rn(__fmul_rn(x[j].v, inv), wn[j]);
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -540,9 +550,10 @@ __device__ __forceinline__ void d1_head(const DkParams& p, const float* src, con
 // exchange buffer, each adds a slice of the outputs in split order and writes it to att. Semantics: src/model.cpp:176-214 of the
 // reference.
 template <int GP>
-__device__ __forceinline__ void d1_attention(const DkParams& p, const int l, const int par, float* scratch, int* dead) {
+__device__ __forceinline__ void d1_attention(const DkParams& p, const int l, const unsigned num, float* scratch, const int* s_pos, int* dead) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x;
-    const int pos = p.pos[p.ctl[0]], T = pos + 1, ns = max(1, min(p.nsplit, (T + D1_SPLIT_KEYS - 1) / D1_SPLIT_KEYS));
+    // (read here, and not kept from layer to layer: what follows from it would take registers from the matvecs)
+    const int pos = *reinterpret_cast<const volatile int*>(s_pos), T = pos + 1, ns = max(1, min(p.nsplit, (T + D1_SPLIT_KEYS - 1) / D1_SPLIT_KEYS));
     if (c >= p.HKV * ns) return;
     const int kvh = c / ns, split = c - kvh * ns, group = p.H / p.HKV, QD = p.H * DK_HD, KD = p.HKV * DK_HD;
     float* const qs = scratch;               // [DK_MAXG][128]
@@ -554,23 +565,27 @@ __device__ __forceinline__ void d1_attention(const DkParams& p, const int l, con
     const int t0 = range_lo(T, ns, split), t1 = range_lo(T, ns, split + 1);  // equal key ranges
     const float* const q_norm = p.norms + size_t(l) * p.norm_stride + 2 * p.E;
     const float2* const cs = reinterpret_cast<const float2*>(p.rope) + size_t(pos) * (p.rope_dim / 2);
-    const float* const qkv = p.ex_q + size_t(par) * p.qkv_len;
-    const int pstride = group * DK_PS;       // floats of one split's partial results
-    const size_t psize = size_t(p.HKV) * p.nsplit * pstride;
-    float* const part = p.ex_s + size_t(kvh) * p.nsplit * pstride;
+    const DkEx* const qkv = p.ex_q;
+    const int pstride = group * DK_PS;       // words of one split's partial results
+    DkEx* const part = p.ex_s + size_t(kvh) * p.nsplit * pstride;
 
     AcKeys<GP, 4, D1_WARPS> keys(kc, vc, size_t(KD), t0, t1, warp, lane);
     keys.first(pos);
     if (warp <= group) {
         const bool key = warp == group;
-        d1_head(p, qkv + (key ? QD + kvh * DK_HD : (kvh * group + warp) * DK_HD), key ? q_norm + DK_HD : q_norm, cs, key ? knew : qs + warp * DK_HD, lane, dead);
+        d1_head(p, qkv + (key ? QD + kvh * DK_HD : (kvh * group + warp) * DK_HD), num, key ? q_norm + DK_HD : q_norm, cs, key ? knew : qs + warp * DK_HD, lane, dead);
     } else if (warp <= GP) *reinterpret_cast<float4*>(qs + (warp - 1) * DK_HD + 4 * lane) = make_float4(0.f, 0.f, 0.f, 0.f);  // heads the group does not have
     if (warp == D1_WARPS - 1) {
-        const float* src = qkv + QD + KD + kvh * DK_HD + 4 * lane;
-        float4 v = ex_ld4(src);
+        const DkEx* src = qkv + QD + KD + kvh * DK_HD + 4 * lane;
+        DkEx v[4];
+        ex_ld2(src, v[0], v[1]);
+        ex_ld2(src + 2, v[2], v[3]);
         Wait wait;
-        while (ex_empty(v) && wait.again(p, dead)) v = ex_ld4(src);
-        *reinterpret_cast<float4*>(vnew + 4 * lane) = v;
+        while ((v[0].num != num || v[1].num != num || v[2].num != num || v[3].num != num) && wait.again(p, dead)) {
+            ex_ld2(src, v[0], v[1]);
+            ex_ld2(src + 2, v[2], v[3]);
+        }
+        *reinterpret_cast<float4*>(vnew + 4 * lane) = make_float4(v[0].v, v[1].v, v[2].v, v[3].v);
     }
     d1_sync();
     if (split == ns - 1 && threadIdx.x < DK_HD) {  // KV append (src/model.cpp:186-189): only row `pos` is written
@@ -580,13 +595,13 @@ __device__ __forceinline__ void d1_attention(const DkParams& p, const int l, con
     d1_stamp(p, l, 12);
     keys.walk(pos, knew, vnew, as, p.scale);
     d1_stamp(p, l, 13);
-    float* const att = p.ex_a;
+    DkEx* const att = p.ex_a;
     ac_finish<GP, 4, D1_WARPS>(keys.w, as, group, warp, lane, [] { d1_sync(); }, [&](int h, int d, float o) {
         if (ns == 1) {
-            ex_put(att, size_t(QD), par, size_t(kvh * group + h) * DK_HD + d, o / as.l[h]);
+            ex_st(att + (kvh * group + h) * DK_HD + d, o / as.l[h], num);
         } else {
-            ex_put(part, psize, par, size_t(split) * pstride + h * DK_PS + d, o);
-            if (d < 2) ex_put(part, psize, par, size_t(split) * pstride + h * DK_PS + DK_HD + d, d ? as.l[h] : as.m[h]);
+            ex_st(part + split * pstride + h * DK_PS + d, o, num);
+            if (d < 2) ex_st(part + split * pstride + h * DK_PS + DK_HD + d, d ? as.l[h] : as.m[h], num);
         }
     });
     if (ns > 1) {
@@ -600,17 +615,18 @@ __device__ __forceinline__ void d1_attention(const DkParams& p, const int l, con
         const int idx = threadIdx.x;
         if (idx < ns * cnt) {
             const int q = idx / cnt, f = f0 + idx - q * cnt, h = f >> 5;
-            const float* src = part + size_t(par) * psize + size_t(q) * pstride + h * DK_PS;
-            float4 o = ex_ld4(src + (f & 31) * 4);
-            float m = ex_ld(src + DK_HD), l2 = ex_ld(src + DK_HD + 1);
+            const DkEx* src = part + q * pstride + h * DK_PS;
+            DkEx o[4], m, l2;
+            auto get = [&] {
+                ex_ld2(src + (f & 31) * 4, o[0], o[1]);
+                ex_ld2(src + (f & 31) * 4 + 2, o[2], o[3]);
+                ex_ld2(src + DK_HD, m, l2);
+            };
+            get();
             Wait wait;
-            while ((ex_empty(o) || ex_empty(m) || ex_empty(l2)) && wait.again(p, dead)) {
-                o = ex_ld4(src + (f & 31) * 4);
-                m = ex_ld(src + DK_HD);
-                l2 = ex_ld(src + DK_HD + 1);
-            }
-            so[idx] = o;
-            sm[idx] = make_float2(m, l2);
+            while ((o[0].num != num || o[1].num != num || o[2].num != num || o[3].num != num || m.num != num || l2.num != num) && wait.again(p, dead)) get();
+            so[idx] = make_float4(o[0].v, o[1].v, o[2].v, o[3].v);
+            sm[idx] = make_float2(m.v, l2.v);
         }
         d1_sync();
 #pragma unroll 1
@@ -625,16 +641,9 @@ __device__ __forceinline__ void d1_attention(const DkParams& p, const int l, con
                 L = fmaf(sm[q * cnt + f].y, w, L);
                 o = fmaf(reinterpret_cast<const float*>(so + q * cnt)[e], w, o);
             }
-            ex_put(att, size_t(QD), par, size_t(kvh * group) * DK_HD + f0 * 4 + e, o / L);
+            ex_st(att + kvh * group * DK_HD + f0 * 4 + e, o / L, num);
         }
     }
-    // Slots that this step does not write may hold words of an earlier step with more keys (one split writes none at all, not
-    // even slot 0): emptied in the first two layers (one half each), before a longer step could take them for its own.
-    if (l < 2)
-#pragma unroll 1
-        for (int q = ns == 1 ? 0 : split + ns; q < p.nsplit; q += ns)
-#pragma unroll 1
-            for (int i = threadIdx.x; i < pstride; i += D1_WORKERS) ex_st(part + size_t(par ^ 1) * psize + size_t(q) * pstride + i, D1_EMPTY);
     d1_sync();  // the scratch area is the next conversion's
 }
 
@@ -675,7 +684,7 @@ __global__ void __launch_bounds__(D1_THREADS, 1) k_decode_one(const __grid_const
     rg.c_off = 0;
     rg.c_seq = rg.freed = 0u;
     rg.freed_out = dk_smem_u32(rshared->freed + wk);
-    if (tid == 0) { s.flags[2] = 0; rshared->producer_done = 0; }
+    if (tid == 0) { s.flags[2] = 0; s.flags[3] = p.pos[p.ctl[0]]; rshared->producer_done = 0; }
     if (tid < D1_WARPS) { rshared->freed[tid] = 0u; rshared->issued[tid] = 0u; }
     if (warp < D1_WARPS && lane < K1_KINDS) {  // this warp's share of every kind of matrix (kinds the model does not have: empty)
         const int kind = lane;
@@ -721,17 +730,17 @@ __global__ void __launch_bounds__(D1_THREADS, 1) k_decode_one(const __grid_const
         }
     }
     int* dead = &s.flags[2];
-    const unsigned step = p.ctl[0], epoch = p.ctl[2];
+    const unsigned num0 = p.ctl[2] * unsigned(p.n_layer) + 1u;  // the number of layer 0's pass: layers are numbered through all launches
     {   // token embedding (get_row, src/ops.cpp:76-82 of the reference): the CTAs decode slices of the row into an exchange buffer
-        const int64_t R = p.token[step];
+        const int64_t R = p.token[p.ctl[0]];
         const int lo = range_lo(p.E, gridDim.x, blockIdx.x), hi = range_lo(p.E, gridDim.x, blockIdx.x + 1);
 #pragma unroll 1
         for (int k = lo + tid; k < hi; k += D1_WORKERS)
-            ex_put(p.ex_e, size_t(p.E), int(epoch & 1u), size_t(k),
-                   p.embd_type == ELB_F16 ? __half2float(reinterpret_cast<const __half*>(p.embd)[R * p.E + k])
-                                          : elem_value(p.embd_type, tiled_elem(p.embd_type, p.embd, p.E, R, k)));
+            ex_st(p.ex_e + k,
+                  p.embd_type == ELB_F16 ? __half2float(reinterpret_cast<const __half*>(p.embd)[R * p.E + k])
+                                         : elem_value(p.embd_type, tiled_elem(p.embd_type, p.embd, p.E, R, k)),
+                  num0);
     }
-    const unsigned n0 = epoch * unsigned(p.n_layer);  // exchanges are numbered through all launches: layer l uses half (n0 + l) & 1
 
     // The step as ONE loop over its matvec stages - per layer q|k|v (0), attn_output (1), gate|up (2), ffn_down (3), then
     // the head (4) - so that conversion, matvec and attention exist once in the kernel.
@@ -741,24 +750,26 @@ __global__ void __launch_bounds__(D1_THREADS, 1) k_decode_one(const __grid_const
     for (int stage = 0; stage < n_stages; ++stage) {
         const bool head = stage + 1 == n_stages;
         const int l = head ? p.n_layer : stage >> 2, k = head ? 4 : stage & 3;
-        const int par = int((n0 + unsigned(l)) & 1u), par_in = k == 0 || head ? par ^ 1 : par;  // (q|k|v and the head read the layer before)
+        const unsigned num = num0 + unsigned(l);
+        const unsigned num_in = (k == 0 || head) && stage > 0 ? num - 1u : num;  // (q|k|v and the head read the layer before)
         if (k == 0) d1_stamp(p, l, 0);
         if (k == 1) {  // attention sits between q|k|v and attn_output
-            d1_attention<GP>(p, l, par, scratch, dead);
+            d1_attention<GP>(p, l, num, scratch, &s.flags[3], dead);
             d1_stamp(p, l, 3);
         }
         const float* const layer_norms = p.norms + size_t(l) * p.norm_stride;  // (not read for the head)
-        const float *A, *B = nullptr, *norm_w = nullptr;
+        const DkEx *A, *B = nullptr;
+        const float* norm_w = nullptr;
         int n = p.E, nl = 4, nm = 1, i0, kind0;
         switch (k) {
             case 0:
-                A = stage == 0 ? p.ex_e + size_t(epoch & 1u) * p.E : p.ex_p2 + size_t(par_in) * 2 * p.E;
+                A = stage == 0 ? p.ex_e : p.ex_p2;
                 norm_w = layer_norms; nl = p.nl_qkv; i0 = 0; kind0 = 0; nm = p.n_qkv;
                 break;
-            case 1: A = p.ex_a + size_t(par) * (p.H * DK_HD); n = p.H * DK_HD; nl = p.nl_wo; i0 = p.n_qkv; kind0 = K1_WO; break;
-            case 2: A = p.ex_p1 + size_t(par) * 2 * p.E; norm_w = layer_norms + p.E; nl = p.nl_gu; i0 = p.n_qkv + 1; kind0 = K1_GU; break;
-            case 3: A = p.ex_g + size_t(par) * p.F; n = p.F; nl = p.nl_down; i0 = p.n_qkv + 2; kind0 = K1_DOWN; nm = p.down_parts; break;
-            default: A = p.ex_p2 + size_t(par_in) * 2 * p.E; norm_w = p.output_norm; i0 = 0; kind0 = K1_HEAD; break;
+            case 1: A = p.ex_a; n = p.H * DK_HD; nl = p.nl_wo; i0 = p.n_qkv; kind0 = K1_WO; break;
+            case 2: A = p.ex_p1; norm_w = layer_norms + p.E; nl = p.nl_gu; i0 = p.n_qkv + 1; kind0 = K1_GU; break;
+            case 3: A = p.ex_g; n = p.F; nl = p.nl_down; i0 = p.n_qkv + 2; kind0 = K1_DOWN; nm = p.down_parts; break;
+            default: A = p.ex_p2; norm_w = p.output_norm; i0 = 0; kind0 = K1_HEAD; break;
         }
         if (norm_w && stage > 0) B = A + p.E;
         int need = 0;
@@ -786,8 +797,8 @@ __global__ void __launch_bounds__(D1_THREADS, 1) k_decode_one(const __grid_const
 #pragma unroll 1
             for (int part = 0; part < parts; ++part) {
                 if (part) d1_sync();  // the activation of the part before has been used
-                if (norm_w) d1_convert<true, F16M>(p, A, B, norm_w, 0, per, nl, act, need, s.red8, rows, dead);
-                else d1_convert<false, F16M>(p, A, nullptr, nullptr, part * per, per, nl, act, need, s.red8, rows, dead);
+                if (norm_w) d1_convert<true, F16M>(p, A, B, num_in, norm_w, 0, per, nl, act, need, s.red8, rows, dead);
+                else d1_convert<false, F16M>(p, A, nullptr, num_in, nullptr, part * per, per, nl, act, need, s.red8, rows, dead);
                 d1_sync();
                 if (part == 0) d1_stamp(p, l, k == 0 ? 1 : 3 * k + 1);
 #pragma unroll 1
@@ -801,18 +812,19 @@ __global__ void __launch_bounds__(D1_THREADS, 1) k_decode_one(const __grid_const
                 inv = float(rsqrt_d(S * p.inv_E + double(p.eps)));
             }
         } else if (norm_w) {
-            d1_keep_rows(p, A, B, rows, k == 0, dead);
+            d1_keep_rows(p, A, B, num_in, rows, dead);
         }
         if (d1_sync_dead(dead)) break;  // (the row sums are in place; all warps agree to stop when a wait has run out)
         if (mine) {
             const int segs = k == 0 ? nm : 1;
 #pragma unroll 1
-            for (int i = 0; i < segs; ++i) d1_epilogue(p, k, kind0 + i, k == 0 ? 1 : nm, i, par, inv, s, s.xrow + kept * p.cta_tiles * 16);
+            for (int i = 0; i < segs; ++i) d1_epilogue(p, k, kind0 + i, k == 0 ? 1 : nm, i, num, inv, s, s.xrow + kept * p.cta_tiles * 16);
         }
         d1_stamp(p, l, k == 0 ? 2 : k == 1 ? 5 : k == 2 ? 8 : 11);
     }
     ring_drain(rg, rshared, warp);  // (nothing is left in flight after a whole step; after a timeout the copies still land here)
     if (tid == 0) {  // the last CTA to finish moves the step on: every CTA has read ctl by then
+        const unsigned step = __ldcg(p.ctl), epoch = __ldcg(p.ctl + 2);
         __threadfence();
         const unsigned old = atomicAdd(p.fin, 1u);
         if (old == gridDim.x - 1) {
@@ -866,12 +878,12 @@ bool decode_one_f16_maps(const DkParams& p, void* host) {
 }
 int decode_one_warps() { return D1_WARPS; }
 
-// Floats of the exchange buffers; sets the pointers of `p` when base is not null (its words empty: all bits set).
-size_t decode_one_exchange(DkParams& p, float* base) {
+// Bytes of the exchange buffers; sets the pointers of `p` when base is not null. All words zero: number 0 is no layer's.
+size_t decode_one_exchange(DkParams& p, uint8_t* base) {
     size_t at = 0;
-    auto take = [&](float** out, size_t n) {
-        if (base) *out = base + at;
-        at += (2 * n + 63) / 64 * 64;
+    auto take = [&](DkEx** out, size_t words) {
+        if (base) *out = reinterpret_cast<DkEx*>(base + at);
+        at += (words * sizeof(DkEx) + 255) / 256 * 256;
     };
     const size_t E = size_t(p.E);
     take(&p.ex_e, E);
@@ -883,6 +895,8 @@ size_t decode_one_exchange(DkParams& p, float* base) {
     take(&p.ex_s, size_t(p.HKV) * p.nsplit * (p.H / p.HKV) * DK_PS);
     return at;
 }
+// Steps after which the numbers of the layers' passes would start again.
+int64_t decode_one_steps(const DkParams& p) { return (int64_t(0xFFFFFFFFu) - 1) / p.n_layer; }
 
 // Bytes per warp ring when the kernel takes all the shared memory a CTA can have (a multiple of 128), capped so that a
 // warp cannot have more than DK_NBAR of the smallest units on request; 0 when not even two of the largest units fit.

@@ -81,7 +81,9 @@ struct Model {
     TpPeerBuf xarea;        // persistent kernel: flags, partial sums and logits, visible to all tensor-parallel ranks
     unsigned* xctl = nullptr;
     bool one = false;            // single GPU: decode_one.cu
-    float* exchange = nullptr;   // its exchange buffers
+    uint8_t* exchange = nullptr; // its exchange buffers
+    size_t exchange_bytes = 0;
+    int64_t one_steps = 0, one_steps_max = 0;  // steps since its layer passes were numbered from 1; most there can be
     uint8_t* f16_maps = nullptr; // its tensor maps (F16 models)
     int8_t* gact = nullptr;  // persistent kernel: limbs of the FFN activation when they do not fit in shared memory
     float* logits_step = nullptr;  // where a single-token step leaves its logits (m->logits unless the persistent kernel runs)
@@ -377,6 +379,11 @@ int body_decode(Model* m) {
 // Enqueue one single-token step on the model's stream (token id and position already on the device). The first
 // step runs eagerly (it also sets the kernels' launch attributes), the second is captured, later ones replay the graph.
 int enqueue_decode_step(Model* m) {
+    if (m->one && m->one_steps++ == m->one_steps_max) {  // the kernel's 32-bit numbers start again, and no word carries one
+        ELB_CUDA(cudaMemsetAsync(m->exchange, 0, m->exchange_bytes, m->stream));
+        ELB_CUDA(cudaMemsetAsync(m->dk.ctl + 2, 0, sizeof(unsigned), m->stream));
+        m->one_steps = 1;
+    }
     if (!m->use_graph || m->decode_calls++ == 0) return body_decode(m);
     if (!m->graph) {
         cudaGraph_t g = nullptr;
@@ -591,10 +598,12 @@ static int setup_decode_one(Model* m) {
         ELB_CUDA(cudaMemcpy(m->f16_maps, maps.data(), maps.size(), cudaMemcpyHostToDevice));
         p.f16_maps = m->f16_maps;
     }
-    const size_t xfloats = decode_one_exchange(p, nullptr);
-    ELB_CUDA(cudaMalloc(&m->exchange, xfloats * sizeof(float)));
-    ELB_CUDA(cudaMemset(m->exchange, 0xFF, xfloats * sizeof(float)));  // every word empty
+    m->exchange_bytes = decode_one_exchange(p, nullptr);
+    ELB_CUDA(cudaMalloc(&m->exchange, m->exchange_bytes));
+    ELB_CUDA(cudaMemset(m->exchange, 0, m->exchange_bytes));
     decode_one_exchange(p, m->exchange);
+    m->one_steps_max = decode_one_steps(p);
+    if (const char* v = std::getenv("ELB_DK_STEPS")) m->one_steps_max = std::max(1, std::atoi(v));  // (tests: a short numbering)
     ELB_CUDA(cudaMalloc(&m->sync_words, 4 * sizeof(unsigned)));
     ELB_CUDA(cudaMemset(m->sync_words, 0, 4 * sizeof(unsigned)));
     ELB_CUDA(cudaMalloc(&m->pos_steps, size_t(m->max_batch) * sizeof(int)));
@@ -1405,6 +1414,14 @@ int model_stats(const Model* m, float* ms, int64_t* launches) {
 int model_hidden(Model* m, float* out) {
     if (!m || !out || !m->finalized) return fail(ELB_ERR_STATE, "hidden: model not ready");
     ELB_CUDA(cudaMemcpy(out, m->x + size_t(m->last_rows - 1) * m->cfg.n_embd, size_t(m->cfg.n_embd) * 4, cudaMemcpyDeviceToHost));
+    return ELB_OK;
+}
+
+int model_fill_exchange(Model* m, int byte) {  // (self-test; between evaluations nothing runs on the model's stream)
+    if (!m || !m->finalized || !m->one) return fail(ELB_ERR_STATE, "selftest: the model does not run on the one-GPU decode kernel");
+    ELB_CUDA(cudaSetDevice(m->device));
+    ELB_CUDA(cudaMemsetAsync(m->exchange, byte, m->exchange_bytes, m->stream));
+    ELB_CUDA(cudaStreamSynchronize(m->stream));
     return ELB_OK;
 }
 

@@ -52,6 +52,11 @@ int elb_device_mem_info(int device, size_t* free_bytes, size_t* total_bytes);
  * up and report: the call returns ELB_ERR_CUDA (elb_last_error names the wait) and the device stays usable; ELB_OK
  * would mean the expiry went unnoticed. Nothing faults or hangs. */
 int elb_selftest_wait_expiry(int device);
+/* Self-test of the decode step on one GPU (no counterpart in the reference): overwrites every word of the buffers through
+ * which its thread blocks hand vectors to each other with `byte`, between two evaluations. No result may depend on what
+ * an earlier step left there. ELB_ERR_STATE when the model does not run on that kernel. */
+struct elb_model;
+int elb_selftest_decode_exchange(struct elb_model* m, int byte);
 
 /* ---- weights ------------------------------------------------------------------------------------------------
  * One weight matrix W[rows][n] in a ggml block format, uploaded and re-laid out for the GPU kernels

@@ -129,6 +129,37 @@ def test_decode_long_and_short_contexts_in_turn(elb, n_layer):
     cpu.close()
 
 
+# the words in the exchange buffers when a step starts - of an earlier step, of another layer, anything that is not numbered
+# for this step - never reach a result: garbage with plausible values between evaluations, and a numbering that starts again
+# after every few steps (the 32-bit numbers of a long-lived model do), give the same bits
+@pytest.mark.parametrize("layout,heads,kv,n_layer", (("q4_k_m", 8, 2, 3), ("f16", 4, 2, 2), ("q8_0", 2, 2, 1)))
+def test_decode_does_not_read_old_exchange_words(elb, monkeypatch, layout, heads, kv, n_layer):
+    from exactinfer_b200 import capi
+    spec = synth.Spec(name="small", n_layer=n_layer, n_embd=512, n_ff=768, n_head=heads, n_head_kv=kv, n_vocab=640, layout=layout,
+                      head_sigma=2e-5)
+    tens = list(synth.generate(spec, 43))
+    toks = synth.lcg_tokens(400, spec.n_vocab, 43)
+    walk = (399, 3, 398, 120, 4, 5, 121, 397)
+
+    def evals(gpu, fill):
+        gpu.eval(toks[:399], 0, want_logits=False)
+        out = []
+        for pos in sorted(walk) + list(walk) * 3:
+            if fill is not None:
+                capi.check(capi.lib().elb_selftest_decode_exchange(gpu._h, fill))
+            out.append(gpu.eval(toks[pos:pos + 1], pos).copy())
+        gpu.close()
+        return out
+
+    want = evals(elb.Backend(spec, tens, 400), None)
+    for fill in (0x3F, 0xBD, 0xFF, 0):  # (four equal bytes as a float: 0.747, -0.0925, NaN, 0; as a number: none that is near)
+        for a, b in zip(evals(elb.Backend(spec, tens, 400), fill), want):
+            assert np.array_equal(a, b), fill
+    monkeypatch.setenv("ELB_DK_STEPS", "3")
+    for a, b in zip(evals(elb.Backend(spec, tens, 400), None), want):
+        assert np.array_equal(a, b)
+
+
 # a feed-forward vector whose limbs (or fp32 values: F16) do not fit in shared memory beside the weight rings: worked off
 # in two and in four parts along k, which every weight format walks with coordinates of its own
 @pytest.mark.parametrize("layout,n_ff", (("q4_k_m", 25600), ("f16", 25600), ("q8_0", 25600), ("q6_k", 25600), ("f16", 57344), ("q4_k_m", 57344)))
