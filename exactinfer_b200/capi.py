@@ -38,6 +38,7 @@ SIGNATURES = {
     "elb_device_mem_info": (C.c_int, [C.c_int, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
     "elb_selftest_wait_expiry": (C.c_int, [C.c_int]),
     "elb_selftest_decode_exchange": (C.c_int, [_vp, C.c_int]),
+    "elb_selftest_decode_plan": (C.c_int, [_i32p, _i32p, C.c_int, C.c_size_t, _i32p]),
     "elb_weight_create": (C.c_int, [C.c_int, C.c_int, C.c_int64, C.c_int64, _vp, C.c_size_t, C.c_int, C.POINTER(_vp)]),
     "elb_weight_destroy": (None, [_vp]),
     "elb_weight_rows": (C.c_int64, [_vp]),

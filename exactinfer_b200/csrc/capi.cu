@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "decode.cuh"
 
 namespace elb {
 static thread_local std::string g_error;
@@ -488,6 +489,10 @@ int elb_model_last_eval_stats(const elb_model* m, float* device_ms, int64_t* ker
     return model_stats(M(m), device_ms, kernel_launches);
 }
 int elb_model_hidden(elb_model* m, float* out) { return model_hidden(M(m), out); }
+int elb_selftest_decode_plan(const int32_t* shape, const int32_t* types, int ctas, size_t smem, int32_t* out) {
+    if (!shape || !types || !out || ctas < 1) return fail(ELB_ERR_INVALID, "selftest: bad argument");
+    return decode_one_selftest_plan(shape, types, ctas, smem, out);
+}
 int elb_selftest_decode_exchange(elb_model* m, int byte) { return model_fill_exchange(M(m), byte); }
 size_t elb_model_weight_bytes(const elb_model* m) { return model_weight_bytes(M(m)); }
 size_t elb_model_kv_bytes_per_token(const elb_model* m) { return model_kv_bytes_per_token(M(m)); }

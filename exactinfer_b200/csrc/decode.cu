@@ -844,6 +844,35 @@ int decode_step_fits(const DkParams& p, int ring_bytes, int device, bool* fits) 
 }
 
 int decode_threads() { return DK_THREADS; }
+void decode_cut_qkv(DkParams& p, const long long* cost) {
+    int tiles = 0;
+    long long sum = 0;
+    for (int i = 0; i < p.n_qkv; ++i) {
+        DkKind& k = p.kind[i];
+        k.group_off = tiles;
+        tiles += k.tiles;
+        k.group_cost = 0;
+        if (!cost) continue;
+        k.cost = int(cost[i] * k.upt);
+        k.group_cost_off = int(sum);
+        sum += (long long)k.cost * k.tiles;
+    }
+    for (int i = 0; i < p.n_qkv; ++i) {
+        p.kind[i].group_tiles = tiles;
+        if (cost && p.n_qkv > 1 && sum < (1ll << 30)) p.kind[i].group_cost = int(sum);
+    }
+}
+
+void decode_extents(const DkParams& p, int grid, int* slots, int* cta_tiles) {
+    *slots = *cta_tiles = 1;
+    for (int i = 0; i < DK_KINDS; ++i) {
+        if (i >= p.n_qkv && i < 3) continue;
+        const CutExtent e = cut_extent(p.kind[i], grid, DK_WARPS);
+        *slots = std::max(*slots, e.warp);
+        *cta_tiles = std::max(*cta_tiles, e.cta);
+    }
+}
+
 int decode_warps() { return DK_WARPS; }
 int decode_max_split() { return DK_MAXSPLIT; }
 int decode_part_stride() { return DK_PS; }

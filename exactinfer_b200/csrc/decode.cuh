@@ -94,16 +94,24 @@ struct DkParams {
     int prof_layer;
 };
 
+// q, k and v (p.kind[0 .. n_qkv), tiles and units set) share one phase: the CTAs cut the tiles of all together, by cost
+// (cost[i]: of a unit) or, with cost null, by count
+void decode_cut_qkv(DkParams& p, const long long* cost);
+// SM clocks of a unit of a block format on a working warp of decode.cu (measured there)
+inline long long decode_unit_cost(int type) { return type == ELB_Q6_K ? 1455 : type == ELB_Q8_0 ? 481 : 875; }
+
 // decode_one.cu (one GPU)
 size_t decode_one_exchange(DkParams& p, uint8_t* base);
 int64_t decode_one_steps(const DkParams& p);
-int decode_one_ring_bytes(const DkParams& p, int max_unit, int min_unit, int device);
+int decode_one_plan(DkParams& p, int grid, int max_unit, int min_unit, size_t smem_optin);
+int decode_one_selftest_plan(const int* shape, const int* types, int ctas, size_t smem, int* out);
 int decode_one_fits(const DkParams& p, int ring_bytes, int device, bool* fits);
 int decode_one_launch(const DkParams& p, int ring_bytes, int grid, cudaStream_t s);
 int decode_one_f16_unit();
 bool decode_one_f16_maps(const DkParams& p, void* host);
-int decode_one_warps();
 
+// decode.cu: most row tiles that a warp's (*slots) and a CTA's (*cta_tiles) share of any matrix touches
+void decode_extents(const DkParams& p, int grid, int* slots, int* cta_tiles);
 // decode.cu (tensor parallelism, and shapes that decode_one.cu does not take)
 // one token at the position / token id stored on the device (step ctl[0] of the arrays); nothing to reset between launches.
 // ring_bytes: size of one warp's ring of weight units in shared memory (decode_ring_bytes); grid: one CTA per SM.

@@ -123,7 +123,7 @@ __device__ __forceinline__ void d1_stamp(const DkParams& p, int l, int ev) {
 enum { K1_WO = 3, K1_GU = 4, K1_HEAD = 5, K1_DOWN = 6, K1_KINDS = K1_DOWN + DK_MAX_PARTS };
 static_assert(K1_KINDS == DK_ONE_KINDS, "tables of the parameter block");
 
-__device__ __forceinline__ const DkKind& d1_whole(const DkParams& p, int kind) { return kind < K1_HEAD ? p.kind[kind] : kind == K1_HEAD ? p.kind[6] : p.kind[5]; }
+__host__ __device__ __forceinline__ const DkKind& d1_whole(const DkParams& p, int kind) { return kind < K1_HEAD ? p.kind[kind] : kind == K1_HEAD ? p.kind[6] : p.kind[5]; }
 // Matrices of a layer in execution order: q|k|v segments, attn_output, gate|up, the parts of ffn_down; layer n_layer: the head.
 __device__ __forceinline__ int d1_kind_of(const DkParams& p, int l, int i) {
     if (l >= p.n_layer) return K1_HEAD;
@@ -876,7 +876,6 @@ bool decode_one_f16_maps(const DkParams& p, void* host) {
         }
     return true;
 }
-int decode_one_warps() { return D1_WARPS; }
 
 // Bytes of the exchange buffers; sets the pointers of `p` when base is not null. All words zero: number 0 is no layer's.
 size_t decode_one_exchange(DkParams& p, uint8_t* base) {
@@ -900,14 +899,73 @@ int64_t decode_one_steps(const DkParams& p) { return (int64_t(0xFFFFFFFFu) - 1) 
 
 // Bytes per warp ring when the kernel takes all the shared memory a CTA can have (a multiple of 128), capped so that a
 // warp cannot have more than DK_NBAR of the smallest units on request; 0 when not even two of the largest units fit.
-int decode_one_ring_bytes(const DkParams& p, int max_unit, int min_unit, int device) {
-    DeviceInfo di;
-    if (device_info(device, &di) != ELB_OK) return 0;
+static int ring_bytes_of(const DkParams& p, int max_unit, int min_unit, size_t smem_optin) {
     const size_t fixed = d1_fixed_smem(p);
-    if (di.smem_optin < fixed + size_t(D1_WARPS) * 2 * max_unit) return 0;
-    size_t per = (di.smem_optin - fixed) / D1_WARPS / 128 * 128;
+    if (smem_optin < fixed + size_t(D1_WARPS) * 2 * max_unit) return 0;
+    size_t per = (smem_optin - fixed) / D1_WARPS / 128 * 128;
     per = std::min(per, size_t(DK_NBAR) * min_unit / 128 * 128);
     return per >= size_t(2) * max_unit ? int(per) : 0;
+}
+
+// How a step's shared memory is used, from the shapes in `p` (kind, n_qkv, E, F, H, HKV, f16): parts of ffn_down, sizes of the
+// activation, of the reduction buffer and of the tables. Returns the bytes of a warp's ring, 0: the shape does not fit.
+// Rings and activation share an SM's memory: ffn_down's activation is worked off in as many equal parts as leave the rings
+// 8 KB per warp (three to four units of weights).
+int decode_one_plan(DkParams& p, int grid, int max_unit, int min_unit, size_t smem_optin) {
+    for (p.down_parts = 1; p.down_parts <= DK_MAX_PARTS; ++p.down_parts) {
+        if (p.kind[5].upt % p.down_parts || (p.F / 256) % p.down_parts) continue;
+        p.n_max = std::max({p.E, p.H * DK_HD, p.F / p.down_parts});
+        p.down_blocks = p.F / 256 / p.down_parts;
+        p.slots = p.cta_tiles = 0;
+        int table = 0, qkv = 0, down = 0;  // entries of the row-tile table; row-tile slots of q|k|v and of the parts, side by side
+        for (int i = 0; i < DK_ONE_KINDS; ++i) {
+            DkKind k = d1_whole(p, i);
+            k.upt = p.upt1[i] = i < K1_DOWN ? k.upt : k.upt / p.down_parts;
+            p.tile_base[i] = table;
+            p.slot_base[i] = 0;
+            if (i < 3 ? i < p.n_qkv : i < K1_DOWN + p.down_parts) {
+                const CutExtent e = cut_extent(k, grid, D1_WARPS);
+                int* side = i < 3 ? &qkv : i >= K1_DOWN ? &down : nullptr;
+                if (side) { p.slot_base[i] = *side; *side += e.warp; }
+                p.slots = std::max(p.slots, p.slot_base[i] + e.warp);
+                table += e.cta;
+                if (i == K1_WO || i == K1_DOWN) p.cta_tiles = std::max(p.cta_tiles, e.cta);  // rows of the residual stream a CTA keeps
+            }
+            p.tile_base[i + 1] = table;
+        }
+        const int ring = ring_bytes_of(p, max_unit, min_unit, smem_optin);
+        if (ring >= std::max(8192, 2 * max_unit)) return ring;
+    }
+    return 0;
+}
+
+// Self-test without a GPU. shape: {n_embd, n_ff, n_head, n_head_kv, n_vocab}; types: block formats of q, k, v, attn_output,
+// gate|up, ffn_down, head; out: {parts of ffn_down, ring bytes, slots per warp, tiles kept}, then the first table entry and the
+// first slot of every kind of matrix (q, k, v, attn_output, gate|up, head, four parts of ffn_down), then the table's length.
+int decode_one_selftest_plan(const int* shape, const int* types, int ctas, size_t smem, int* out) {
+    DkParams p{};
+    p.E = shape[0]; p.F = shape[1]; p.H = shape[2]; p.HKV = shape[3]; p.n_qkv = 3;
+    p.f16 = types[6] == ELB_F16;
+    const int QD = p.H * DK_HD, KD = p.HKV * DK_HD, rows[7] = {QD, KD, KD, p.E, 2 * p.F, p.E, shape[4]}, n[7] = {p.E, p.E, p.E, QD, p.E, p.F, p.E};
+    int unit_max = 0, unit_min = 1 << 30;
+    long long cost[3];
+    for (int i = 0; i < 7; ++i) {
+        const int tiles = (rows[i] + 15) / 16, upt = n[i] / (types[i] == ELB_F16 || types[i] == ELB_Q8_0 ? 128 : 256);
+        const int ub = types[i] == ELB_F16 ? D1_F16_UNIT : types[i] == ELB_Q4_K ? Q4K_UNIT : types[i] == ELB_Q6_K ? Q6K_UNIT : Q8_UNIT;
+        p.kind[i] = DkKind{tiles, upt, rows[i], n[i], tiles, 0, 0, 0};
+        p.kind[i].balanced = (i == 3 || i == 5) && tiles >= ctas;
+        if (i < 3) cost[i] = decode_unit_cost(types[i]);
+        unit_max = std::max(unit_max, ub);
+        unit_min = std::min(unit_min, ub);
+    }
+    decode_cut_qkv(p, cost);
+    out[1] = decode_one_plan(p, ctas, unit_max, unit_min, smem);
+    out[0] = out[1] ? p.down_parts : 0;
+    out[2] = p.slots;
+    out[3] = p.cta_tiles;
+    for (int i = 0; i < DK_ONE_KINDS; ++i) { out[4 + i] = p.tile_base[i]; out[4 + DK_ONE_KINDS + i] = p.slot_base[i]; }
+    out[4 + 2 * DK_ONE_KINDS] = p.tile_base[DK_ONE_KINDS];
+    return ELB_OK;
 }
 
 int decode_one_launch(const DkParams& p, int ring_bytes, int grid, cudaStream_t s) {

@@ -135,15 +135,14 @@ __device__ __forceinline__ int kind_li(const DkParams& p, int l, int i) { return
 // Whole tiles of the matrix's group by default (no tile is shared between CTAs: the phase ends without any exchange;
 // a group with fewer tiles than CTAs occupies the first CTAs only); equal unit ranges for a balanced matrix.
 struct WarpRange { int cA, cB, wA, wB; };
-static __device__ __noinline__ WarpRange warp_range(const DkKind& m, int warp, int warps = DK_WARPS) {
-    const int c = blockIdx.x;
+__host__ __device__ inline WarpRange cut_range(const DkKind& m, int c, int ctas, int warp, int warps) {
     WarpRange r;
     if (m.balanced) {
         const int U = m.tiles * m.upt;
-        r.cA = range_lo(U, gridDim.x, c);
-        r.cB = range_lo(U, gridDim.x, c + 1);
+        r.cA = range_lo(U, ctas, c);
+        r.cB = range_lo(U, ctas, c + 1);
     } else {
-        const int G = min(int(gridDim.x), m.group_tiles);
+        const int G = min(ctas, m.group_tiles);
         if (m.group_cost > 0) {  // CTA c takes the tiles whose cost position lies in [C c / G, C (c + 1) / G)
             auto bound = [&](int cc) {  // first tile of this matrix at or behind the cost position of boundary cc
                 const long long rel = (long long)m.group_cost * cc / G - m.group_cost_off;
@@ -160,6 +159,24 @@ static __device__ __noinline__ WarpRange warp_range(const DkKind& m, int warp, i
     r.wA = r.cA + range_lo(r.cB - r.cA, warps, warp);
     r.wB = r.cA + range_lo(r.cB - r.cA, warps, warp + 1);
     return r;
+}
+static __device__ __noinline__ WarpRange warp_range(const DkKind& m, int warp, int warps = DK_WARPS) {
+    return cut_range(m, int(blockIdx.x), int(gridDim.x), warp, warps);
+}
+
+// Most row tiles that the share of a CTA, and of one of its warps, touches. Taken from the cut itself: q, k and v are cut as
+// one group and by cost, so that a CTA can hold many more tiles of a cheap format than its share by count.
+struct CutExtent { int cta, warp; };
+inline CutExtent cut_extent(const DkKind& m, int ctas, int warps) {
+    CutExtent e{0, 1};
+    auto touched = [&](int a, int b) { return a < b ? (b - 1) / m.upt - a / m.upt + 1 : 0; };
+    for (int c = 0; c < ctas; ++c)
+        for (int w = 0; w < warps; ++w) {
+            const WarpRange r = cut_range(m, c, ctas, w, warps);
+            if (w == 0) e.cta = max(e.cta, touched(r.cA, r.cB));
+            e.warp = max(e.warp, touched(r.wA, r.wB));
+        }
+    return e;
 }
 
 // The shares of a warp (and of its CTA) in the matrices of every kind are computed once, when the kernel starts, and

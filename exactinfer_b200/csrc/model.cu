@@ -493,14 +493,9 @@ static int setup_decode_one(Model* m) {
         unit_min = std::min(unit_min, ub);
     };
     const Layer& L0 = m->layers[0];
-    int group_tiles = 0;
-    for (size_t i = 0; i < nq; ++i) group_tiles += int(L0.qkv[i].w->tiles);
-    for (size_t i = 0, off = 0; i < nq; ++i) {  // q, k, v share one phase: the CTAs cut the tiles of all three together
+    for (size_t i = 0; i < nq; ++i) {
         p.kind[i] = kind_of(L0.qkv[i].w);
-        p.kind[i].group_tiles = group_tiles;
-        p.kind[i].group_off = int(off);
         p.qkv_col[i] = int(L0.qkv[i].col);
-        off += size_t(L0.qkv[i].w->tiles);
     }
     p.kind[3] = kind_balanced(L0.wo); p.kind[4] = kind_of(L0.gu); p.kind[5] = kind_balanced(L0.down); p.kind[6] = kind_of(m->head);
     for (int l = 0; l < L; ++l) {
@@ -518,22 +513,15 @@ static int setup_decode_one(Model* m) {
     p.W[L][0] = m->head->tiled;
     p.wtype[L][0] = uint8_t(m->head->type);
     account(m->head);
-    if (nq > 1) {  // q|k|v cut by cost: a tile's units times the time a unit of its format takes
-        auto unit_cost = [](int type) { return type == ELB_Q6_K ? 1455 : type == ELB_Q8_0 ? 481 : 875; };  // SM clocks, measured
-        long long off = 0;
-        for (size_t i = 0; i < nq; ++i) {
-            long long sum = 0;
-            for (int l = 0; l < L; ++l) sum += unit_cost(p.wtype[l][i]);
-            p.kind[i].cost = int(sum / L) * p.kind[i].upt;
-            p.kind[i].group_cost_off = int(off);
-            off += (long long)p.kind[i].cost * p.kind[i].tiles;
-        }
-        if (off < (1ll << 30))
-            for (size_t i = 0; i < nq; ++i) p.kind[i].group_cost = int(off);
+    p.n_layer = L; p.n_qkv = int(nq);
+    long long cost[3] = {};
+    for (size_t i = 0; i < nq; ++i) {
+        for (int l = 0; l < L; ++l) cost[i] += decode_unit_cost(p.wtype[l][i]);
+        cost[i] /= L;
     }
+    decode_cut_qkv(p, cost);
     for (int i = 0; i < 7; ++i)  // 32-bit unit arithmetic in the kernel
         if (int64_t(p.kind[i].tiles) * p.kind[i].upt * di.sm_count >= (int64_t(1) << 31)) return ELB_OK;
-    p.n_layer = L; p.n_qkv = int(nq);
     p.norms = m->norm_arena;
     p.norm_stride = int(2 * E + 2 * c.head_dim);
     p.kc = m->kcache; p.vc = m->vcache;  // sequence 0
@@ -549,45 +537,9 @@ static int setup_decode_one(Model* m) {
     p.rope = m->rope; p.x = m->x;
     p.logits_peer[0] = m->logits;
     if (m->HKV > di.sm_count || group > 8) return ELB_OK;
-    // Rings and activation share an SM's memory: ffn_down's activation is worked off in as many equal parts as leave the
-    // rings 8 KB per warp (three to four units of weights).
-    const int min_ring = std::max(8192, 2 * unit_max);
     bool fits = false;
-    for (p.down_parts = 1; p.down_parts <= DK_MAX_PARTS && !fits; ++p.down_parts) {
-        if (p.kind[5].upt % p.down_parts || (F / 256) % p.down_parts) continue;
-        p.n_max = std::max({E, QD, F / p.down_parts});
-        // row-tile slots of the reduction buffer: what one warp's share of each kind can touch; kinds of a stage side by side
-        auto slots_of = [&](const DkKind& k, int u) {
-            const int64_t per_cta = (int64_t(k.tiles) + di.sm_count - 1) / di.sm_count * u, per_warp = (per_cta + decode_one_warps() - 1) / decode_one_warps();
-            return int((per_warp + u - 1) / u + 2);
-        };
-        int used = 0, most = 0, tiles = 0;
-        for (size_t i = 0; i < nq; ++i) {
-            p.slot_base[i] = used;
-            // (by cost a CTA can have more tiles of a cheap format than its share by count)
-            used += 2 * slots_of(p.kind[i], p.kind[i].upt);
-        }
-        most = used;
-        p.slot_base[3] = p.slot_base[4] = p.slot_base[5] = 0;
-        most = std::max({most, slots_of(p.kind[3], p.kind[3].upt), slots_of(p.kind[4], p.kind[4].upt), slots_of(p.kind[6], p.kind[6].upt)});
-        used = 0;
-        for (int h = 0; h < p.down_parts; ++h) { p.slot_base[6 + h] = used; used += slots_of(p.kind[5], p.kind[5].upt / p.down_parts); }
-        p.slots = std::max(most, used);
-        p.down_blocks = F / 256 / p.down_parts;
-        for (int i = 0, at = 0; i < DK_ONE_KINDS; ++i) {
-            const DkKind& k = p.kind[i < 5 ? i : i == 5 ? 6 : 5];
-            p.upt1[i] = i < 6 ? k.upt : k.upt / p.down_parts;
-            p.tile_base[i] = at;
-            at += ((k.tiles + di.sm_count - 1) / di.sm_count + 2) * (i < 3 ? 3 : 1);
-            p.tile_base[i + 1] = at;
-        }
-        for (int i : {3, 5}) tiles = std::max(tiles, (p.kind[i].tiles + di.sm_count - 1) / di.sm_count + 2);
-        p.cta_tiles = tiles;  // of the row-parallel matrices: rows of the residual stream a CTA keeps
-        m->dk_slot = decode_one_ring_bytes(p, unit_max, unit_min, m->device);
-        if (m->dk_slot < min_ring) continue;
-        ELB_TRY(decode_one_fits(p, m->dk_slot, m->device, &fits));
-        if (fits) break;
-    }
+    m->dk_slot = decode_one_plan(p, di.sm_count, unit_max, unit_min, di.smem_optin);
+    if (m->dk_slot) ELB_TRY(decode_one_fits(p, m->dk_slot, m->device, &fits));
     int coop = 0;
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->device) != cudaSuccess) { cudaGetLastError(); coop = 0; }
     if (!fits || !coop) return ELB_OK;
@@ -687,16 +639,11 @@ int setup_decode_kernel(Model* m, bool local_ok = true) {
     account(m->head);
     for (int l = 0; l < c.n_layer; ++l) {
         const Layer& L = m->layers[size_t(l)];
-        int group = 0;
-        for (size_t i = 0; i < nq; ++i) group += int(L.qkv[i].w->tiles);
-        for (size_t i = 0, off = 0; i < nq; ++i) {  // q, k, v share one phase: the CTAs cut the tiles of all three together
+        for (size_t i = 0; i < nq; ++i) {
             if (l == 0) {
                 p.kind[i] = kind_of(L.qkv[i].w);
-                p.kind[i].group_tiles = group;
-                p.kind[i].group_off = int(off);
                 p.qkv_col[i] = int(L.qkv[i].col);
             }
-            off += size_t(L.qkv[i].w->tiles);
             p.W[l][i] = L.qkv[i].w->tiled;
             p.wtype[l][i] = uint8_t(L.qkv[i].w->type);
             account(L.qkv[i].w);
@@ -709,18 +656,18 @@ int setup_decode_kernel(Model* m, bool local_ok = true) {
             account(rest[i]);
         }
     }
-    if (nq > 1 && !env_on("ELB_DK_EVEN_TILES")) {  // q|k|v cut by cost: a tile's units times the time a unit of its format takes
-        auto unit_cost = [](int type) { return type == ELB_Q6_K ? 1455 : type == ELB_Q8_0 ? 481 : 875; };  // SM clocks, measured
-        long long off = 0;
-        for (size_t i = 0; i < nq; ++i) {
-            long long sum = 0;
-            for (int l = 0; l < c.n_layer; ++l) sum += unit_cost(p.wtype[l][i]);
-            p.kind[i].cost = int(sum / c.n_layer) * p.kind[i].upt;
-            p.kind[i].group_cost_off = int(off);
-            off += (long long)p.kind[i].cost * p.kind[i].tiles;
-        }
-        if (off < (1ll << 30))
-            for (size_t i = 0; i < nq; ++i) p.kind[i].group_cost = int(off);
+    p.n_qkv = int(nq);
+    long long cost[3] = {};
+    for (size_t i = 0; i < nq; ++i) {
+        for (int l = 0; l < c.n_layer; ++l) cost[i] += decode_unit_cost(p.wtype[l][i]);
+        cost[i] /= c.n_layer;
+    }
+    decode_cut_qkv(p, env_on("ELB_DK_EVEN_TILES") ? nullptr : cost);
+    {   // (at least the sizes above, which do not depend on the cut of q|k|v)
+        int warp_most = 0, cta_most = 0;
+        decode_extents(p, di.sm_count, &warp_most, &cta_most);
+        slots = std::max(slots, warp_most);
+        cta_tiles = std::max(cta_tiles, cta_most);
     }
     p.norms = m->norm_arena;
     p.norm_stride = int(2 * E + 2 * c.head_dim);
@@ -763,7 +710,7 @@ int setup_decode_kernel(Model* m, bool local_ok = true) {
         return ELB_OK;
     };
     int rc_local = local_words();  // a failure is carried to the agreement below, not returned before it
-    p.n_layer = c.n_layer; p.n_qkv = int(nq);
+    p.n_layer = c.n_layer;
     p.output_norm = m->output_norm;
     p.embd = m->embd->tiled; p.embd_type = m->embd->type;
     p.E = E; p.F = F; p.H = m->H; p.HKV = m->HKV; p.rope_dim = c.rope_dim; p.n_ctx = m->n_ctx;

@@ -57,6 +57,12 @@ int elb_selftest_wait_expiry(int device);
  * an earlier step left there. ELB_ERR_STATE when the model does not run on that kernel. */
 struct elb_model;
 int elb_selftest_decode_exchange(struct elb_model* m, int byte);
+/* Self-test without a GPU: how that step is laid out for a shape {n_embd, n_ff, n_head, n_head_kv, n_vocab} in the block formats
+ * `types` {q, k, v, attn_output, gate|up, ffn_down, head} on `ctas` thread blocks with `smem` bytes of shared memory each.
+ * out, 25 numbers: parts ffn_down is worked off in along k (0: the shape does not fit), ring bytes of a warp, row-tile slots
+ * of a warp, row tiles kept, first entry of each kind of matrix (q, k, v, attn_output, gate|up, head, four parts of
+ * ffn_down) in the table of a thread block's row tiles, first slot of each kind, length of the table. */
+int elb_selftest_decode_plan(const int32_t* shape, const int32_t* types, int ctas, size_t smem, int32_t* out);
 
 /* ---- weights ------------------------------------------------------------------------------------------------
  * One weight matrix W[rows][n] in a ggml block format, uploaded and re-laid out for the GPU kernels

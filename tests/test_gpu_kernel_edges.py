@@ -129,6 +129,31 @@ def test_decode_long_and_short_contexts_in_turn(elb, n_layer):
     cpu.close()
 
 
+# more query heads than the built-in shapes have, q and v in a costlier format than k: one thread block gets ten row tiles of k
+# alone, more than three times k's share by count
+def test_decode_uneven_cut_of_qkv(elb):
+    spec = synth.Spec(name="small", n_layer=2, n_embd=512, n_ff=512, n_head=96, n_head_kv=12, n_vocab=512, layout="q4_k_m",
+                      head_sigma=2e-5)
+    tens = []
+    rng = np.random.default_rng(5)
+    for role, layer, t, rows, n, data in synth.generate(spec, 37):
+        want = {"attn_q": synth.Q6_K, "attn_k": synth.Q4_K, "attn_v": synth.Q6_K}.get(role, t)
+        if want != t:
+            data = synth.rand_weight(rng, want, rows, n)
+        tens.append((role, layer, want, rows, n, data))
+    toks = synth.lcg_tokens(150, spec.n_vocab, 37)
+    gpu, cpu = elb.Backend(spec, tens, 160), ol.OracleModel(spec, tens, 160)
+    gpu.eval(toks[:140], 0, want_logits=False)
+    cpu.eval(toks[:140], 0)
+    for pos in (0, 139, 140, 141):
+        a, b = gpu.eval(toks[pos:pos + 1], pos), cpu.eval(toks[pos:pos + 1], pos)
+        assert gpu.last_eval_stats()[1] == 1, "the persistent kernel must run"
+        assert np.abs(a - b).max() <= 2e-4 * np.abs(b).max()
+        assert np.array_equal(a, gpu.eval(toks[pos:pos + 1], pos))
+    gpu.close()
+    cpu.close()
+
+
 # the words in the exchange buffers when a step starts - of an earlier step, of another layer, anything that is not numbered
 # for this step - never reach a result: garbage with plausible values between evaluations, and a numbering that starts again
 # after every few steps (the 32-bit numbers of a long-lived model do), give the same bits
@@ -161,8 +186,9 @@ def test_decode_does_not_read_old_exchange_words(elb, monkeypatch, layout, heads
 
 
 # a feed-forward vector whose limbs (or fp32 values: F16) do not fit in shared memory beside the weight rings: worked off
-# in two and in four parts along k, which every weight format walks with coordinates of its own
-@pytest.mark.parametrize("layout,n_ff", (("q4_k_m", 25600), ("f16", 25600), ("q8_0", 25600), ("q6_k", 25600), ("f16", 57344), ("q4_k_m", 57344)))
+# in two and in four parts along k, which every weight format walks with coordinates of its own (test_decode_plan_cpu.py says
+# how many parts a length gives)
+@pytest.mark.parametrize("layout,n_ff", (("q4_k_m", 25600), ("f16", 25600), ("q8_0", 25600), ("q6_k", 25600), ("f16", 28672), ("f16", 57344), ("q4_k_m", 57344)))
 def test_decode_long_feed_forward(elb, layout, n_ff):
     spec = synth.Spec(name="small", n_layer=2, n_embd=256, n_ff=n_ff, n_head=2, n_head_kv=1, n_vocab=640, layout=layout,
                       head_sigma=2e-5)
