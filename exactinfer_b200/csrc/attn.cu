@@ -715,11 +715,12 @@ __global__ void __launch_bounds__(TP_THREADS) k_logits_top(const float* __restri
     mx = red_f[0];
 #pragma unroll
     for (int w = 1; w < TP_WARPS; ++w) mx = fmaxf(mx, red_f[w]);
+    const double from = mx == -INFINITY ? 0.0 : double(mx);  // (no finite logit: the sum is then 0, or NaN if one of them is)
     double sum = 0.0;
 #pragma unroll 1
     for (int j = 0; j < TP_PER; ++j) {
         const int i = base + j * TP_THREADS;
-        if (i < n) sum += exp(double(__ldcg(logits + i)) - double(mx));
+        if (i < n) sum += exp(double(__ldcg(logits + i)) - from);
     }
     sum = warp_sum(sum);
     if (lane == 0) red_d[warp] = sum;
@@ -767,10 +768,7 @@ __global__ void __launch_bounds__(TP_THREADS) k_logits_top(const float* __restri
         for (int i = lane; i < chunks; i += 32) M = fmaxf(M, __ldcg(&parts[i].mx));
         M = warp_max(M);
         double t = 0.0;
-        for (int i = lane; i < chunks; i += 32) {
-            const float m = __ldcg(&parts[i].mx);
-            if (m != -INFINITY || M == -INFINITY) t += __ldcg(&parts[i].sum) * exp(double(m) - double(M));
-        }
+        for (int i = lane; i < chunks; i += 32) t += __ldcg(&parts[i].sum) * exp(double(__ldcg(&parts[i].mx)) - double(M));
         t = warp_sum(t);
         if (lane == 0) *reinterpret_cast<double*>(out) = double(M) + log(t);
     }

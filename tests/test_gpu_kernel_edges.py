@@ -74,6 +74,41 @@ def test_top_tokens_at_chunk_edges(elb, vocab):
     gpu.close()
 
 
+# rows of logits that a broken model gives: one chunk of the reduction (and a part of one) without any finite logit
+@pytest.mark.parametrize("lo,hi", ((2560, 5120), (0, 2560), (7680, 7681), (100, 200)))
+@pytest.mark.parametrize("what", ("nan", "-inf", "both"))
+def test_log_sum_exp_with_nan_and_infinity(elb, lo, hi, what):
+    spec = synth.Spec(name="small", n_layer=1, n_embd=256, n_ff=512, n_head=4, n_head_kv=2, n_vocab=7681, layout="f16", head_sigma=1e-2)
+    tens = list(synth.generate(spec, 5))
+    tok = np.array([6000], np.int32)
+
+    def logits_with(inf):  # one weight of the rows is +-infinity or NaN, the others are 0
+        role, layer, t, rows, n, emb = tens[0]
+        half = emb.copy().view(np.uint16).reshape(rows, n)
+        half[lo:hi] = 0
+        half[lo:hi, 0] = 0x7E00 if what == "nan" else inf
+        if what == "both":
+            half[lo:hi:2, 0] = 0x7E00
+        gpu = elb.Backend(spec, [(role, layer, t, rows, n, half.view(np.uint8).reshape(rows, -1))] + tens[1:], 8)
+        full = gpu.eval(tok, 0)
+        return (full.copy(), *gpu.eval_top(tok, 0, k=5))
+
+    for inf in (0x7C00, 0xFC00):  # (the sign of the activation decides which of them gives -infinity)
+        full, ids, vals, lse = logits_with(inf)
+        if not np.isposinf(full).any():
+            break
+    bad = full[lo:hi]
+    assert (np.isnan(bad) if what == "nan" else np.isneginf(bad) if what == "-inf" else ~np.isfinite(bad)).all()
+    assert np.isfinite(np.delete(full, np.s_[lo:hi])).all()
+    if what == "-inf":
+        want = ol.logsumexp(full)
+        assert np.isfinite(want) and abs(lse - want) <= 1e-12 * max(1.0, abs(want))
+    else:
+        assert np.isnan(lse)
+    order = np.argsort(-np.where(np.isnan(full), -np.inf, full).astype(np.float64), kind="stable")[:5]
+    assert np.array_equal(ids, order) and np.array_equal(vals, full[order])
+
+
 def decode_pair(elb, spec, seed, n_ctx, walk):
     """Single-token evaluations at the positions of `walk` (rows in front of them filled by prompt chunks), against the
     CPU oracle on the same cache contents; every evaluation twice, which must give the same bits."""
