@@ -19,8 +19,9 @@ int fail(int code, const std::string& msg) {
 namespace {
 // Device scratch of the operator entry points, kept between calls: cudaMalloc + cudaFree (which waits for the device and
 // unmaps) cost 0.6-3 ms per call of a 37-row matmul whose kernels take 20 us. A buffer belongs to one call from alloc()
-// to the end of its scope, which every entry point reaches after its own synchronize, so calls on other threads and
-// streams never meet in one. Bounded: at most SCRATCH_KEEP idle buffers and SCRATCH_BYTES in all stay per device; the
+// to the end of its scope. It goes back to the pool only from a call that has waited for all it enqueued (settled()), so
+// calls on other threads and streams never meet in one; a call that fails in between frees its buffers, which waits for the
+// device. Bounded: at most SCRATCH_KEEP idle buffers and SCRATCH_BYTES in all stay per device; the
 // rest, and everything when the last weight of the device goes or an allocation fails, is given back to the driver.
 constexpr size_t SCRATCH_KEEP = 6, SCRATCH_BYTES = size_t(256) << 20;
 struct Scratch {
@@ -87,7 +88,11 @@ struct Dev {
     void* p = nullptr;
     size_t bytes = 0;
     int device = 0;
-    ~Dev() { if (p) scratch_of(device).give(p, bytes); }
+    bool settled = false;  // the device is done with the buffer
+    ~Dev() {
+        if (p && settled) scratch_of(device).give(p, bytes);
+        else if (p) cudaFree(p);
+    }
     int alloc(size_t n) {  // on the current device
         ELB_CUDA(cudaGetDevice(&device));
         n = (std::max<size_t>(n, 16) + 511) / 512 * 512;
@@ -107,6 +112,10 @@ struct Dev {
     }
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
+template <class... D> int settled(D&... d) {  // after the call's last wait
+    ((d.settled = true), ...);
+    return ELB_OK;
+}
 }  // namespace
 }  // namespace elb
 
@@ -211,7 +220,7 @@ int elb_get_rows(const elb_weight* w, int64_t row0, int64_t count, float* out) {
     ELB_TRY(d.alloc(size_t(count) * W(w)->n * 4));
     ELB_TRY(elb_get_rows_dev(w, row0, count, d.as<float>()));
     ELB_CUDA(cudaMemcpy(out, d.p, size_t(count) * W(w)->n * 4, cudaMemcpyDeviceToHost));
-    return ELB_OK;
+    return settled(d);
 }
 
 // split (quantized weights) + matvec on stream s; dbg may carry the parity dump pointers
@@ -243,7 +252,7 @@ int elb_matvec(const elb_weight* w, const float* x, float* y, int nl) {
     ELB_CUDA(cudaMemcpy(dx.p, x, size_t(W(w)->n) * 4, cudaMemcpyHostToDevice));
     ELB_TRY(elb_matvec_dev(w, dx.as<float>(), dy.as<float>(), nl));
     ELB_CUDA(cudaMemcpy(y, dy.p, size_t(W(w)->rows) * 4, cudaMemcpyDeviceToHost));
-    return ELB_OK;
+    return settled(dx, dy);
 }
 
 static int matmul_dev_on(const Weight* w, const float* d_x, int64_t b, float* d_y, int nl, cudaStream_t s, Dev* scratch) {
@@ -293,6 +302,7 @@ int elb_matmul_acc(const elb_weight* w, const float* x, int64_t b, int nl, int32
     ELB_TRY(split_launch(dx.as<float>(), ww->n, b, int(ww->n), nl, nullptr, 0.f, limbs, inv, xs, nullptr));
     ELB_TRY(gemm_tc_launch(ww, limbs, inv, xs, int(b), nl, dy.as<float>(), ww->rows, nullptr, EPI_STORE, nullptr, false, dA.as<int32_t>()));
     ELB_CUDA(cudaStreamSynchronize(nullptr));
+    settled(dx, dy, scratch, dA);
     ELB_TRY(gemm_tc_check());
     std::vector<int32_t> tmp(nA);
     ELB_CUDA(cudaMemcpy(tmp.data(), dA.p, nA * 4, cudaMemcpyDeviceToHost));
@@ -307,6 +317,7 @@ int elb_matmul_dev(const elb_weight* w, const float* d_x, int64_t b, float* d_y,
     Dev scratch;
     ELB_TRY(matmul_dev_on(W(w), d_x, b, d_y, nl, nullptr, &scratch));
     ELB_CUDA(cudaStreamSynchronize(nullptr));
+    settled(scratch);
     ELB_TRY(gemm_f16_tc_check());
     return gemm_tc_check();
 }
@@ -320,7 +331,7 @@ int elb_matmul(const elb_weight* w, const float* x, int64_t b, float* y, int nl)
     ELB_CUDA(cudaMemcpy(dx.p, x, size_t(b) * W(w)->n * 4, cudaMemcpyHostToDevice));
     ELB_TRY(elb_matmul_dev(w, dx.as<float>(), b, dy.as<float>(), nl));
     ELB_CUDA(cudaMemcpy(y, dy.p, size_t(b) * W(w)->rows * 4, cudaMemcpyDeviceToHost));
-    return ELB_OK;
+    return settled(dx, dy);
 }
 
 int elb_rmsnorm(float* out, const float* x, const float* w, int n, float eps, int rows) {
@@ -334,7 +345,7 @@ int elb_rmsnorm(float* out, const float* x, const float* w, int n, float eps, in
     ELB_CUDA(cudaMemcpy(dw.p, w, size_t(n) * 4, cudaMemcpyHostToDevice));
     ELB_TRY(rmsnorm_launch(dy.as<float>(), dx.as<float>(), dw.as<float>(), n, eps, rows, nullptr));
     ELB_CUDA(cudaMemcpy(out, dy.p, size_t(rows) * n * 4, cudaMemcpyDeviceToHost));
-    return ELB_OK;
+    return settled(dx, dw, dy);
 }
 
 int elb_split_limbs(int device, const float* x, int64_t b, int64_t n, int nl, int8_t* limbs, float* inv_scale) {
@@ -349,7 +360,7 @@ int elb_split_limbs(int device, const float* x, int64_t b, int64_t n, int nl, in
     ELB_TRY(split_launch(dx.as<float>(), n, b, int(n), nl, nullptr, 0.f, dl.as<int8_t>(), di.as<float>(), nullptr, nullptr));
     ELB_CUDA(cudaMemcpy(limbs, dl.p, size_t(nl) * b * n, cudaMemcpyDeviceToHost));
     ELB_CUDA(cudaMemcpy(inv_scale, di.p, size_t(b) * 4, cudaMemcpyDeviceToHost));
-    return ELB_OK;
+    return settled(dx, dl, di);
 }
 
 int elb_limb_sums(const elb_weight* w, const float* x, int nl, int32_t* P, int32_t* I, int32_t* J) {
@@ -372,6 +383,7 @@ int elb_limb_sums(const elb_weight* w, const float* x, int nl, int32_t* P, int32
     a.dbgP = dP.as<int32_t>(); a.dbgI = dI.as<int32_t>(); a.dbgJ = dJ.as<int32_t>();
     ELB_TRY(matvec_on(ww, dx.as<float>(), dy.as<float>(), nl, nullptr, &a));
     ELB_CUDA(cudaStreamSynchronize(nullptr));
+    settled(dx, dy, dP, dI, dJ);
     // device arrays carry 4 limb slots; compact to nl
     auto fetch = [&](int32_t* dst, const Dev& src, size_t n4) -> int {
         if (!dst) return ELB_OK;
@@ -566,6 +578,7 @@ int elb_bench_matmul(elb_weight* const* ws, int n_w, const float* d_x, int64_t b
     for (int i = 0; i < iters && rc == ELB_OK; ++i) rc = matmul_dev_on(W(ws[i % n_w]), d_x, b, d_y, nl, s, &scratch);
     cudaEventRecord(e1, s);
     const cudaError_t e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) settled(scratch);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);

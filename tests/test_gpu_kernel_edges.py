@@ -54,6 +54,32 @@ def test_operator_scratch_is_reused_and_given_back(elb):
     assert free() >= before
 
 
+def test_operator_scratch_of_a_failed_call_is_not_kept(elb):
+    """A call that fails behind a launch has not waited for it: its scratch is freed, which does, and not given to the next."""
+    import ctypes as C
+    from exactinfer_b200 import capi
+
+    def free():
+        f, t = C.c_size_t(), C.c_size_t()
+        capi.check(capi.lib().elb_device_mem_info(0, C.byref(f), C.byref(t)))
+        return f.value
+
+    rng = np.random.default_rng(2)
+    w = elb.Weight(synth.Q4_K, 64, 4096, synth.rand_weight(rng, synth.Q4_K, 64, 4096))  # no digit planes: refused behind the split
+    x, y = C.c_void_p(), C.c_void_p()
+    capi.check(capi.lib().elb_malloc(0, 512 * 4096 * 4, C.byref(x)))
+    capi.check(capi.lib().elb_malloc(0, 512 * 64 * 4, C.byref(y)))
+    capi.check(capi.lib().elb_memcpy_h2d(x, rng.normal(size=512 * 4096).astype(np.float32).ctypes.data_as(C.c_void_p), 512 * 4096 * 4))
+    w.matvec(np.zeros(4096, np.float32))
+    before = free()
+    for _ in range(3):
+        assert capi.lib().elb_matmul_dev(w._h, x, 512, y, 4) == capi.ERR_STATE
+    assert free() == before  # 8 MB of limbs otherwise
+    for p in (x, y):
+        capi.check(capi.lib().elb_free(p))
+    w.close()
+
+
 # vocabularies below, at and just past a chunk of the reduction (2560 logits), and of several chunks
 @pytest.mark.parametrize("vocab", (64, 2559, 2560, 2561, 7681))
 def test_top_tokens_at_chunk_edges(elb, vocab):
