@@ -21,8 +21,9 @@ namespace {
 // unmaps) cost 0.6-3 ms per call of a 37-row matmul whose kernels take 20 us. A buffer belongs to one call from alloc()
 // to the end of its scope. It goes back to the pool only from a call that has waited for all it enqueued (settled()), so
 // calls on other threads and streams never meet in one; a call that fails in between frees its buffers, which waits for the
-// device. Bounded: at most SCRATCH_KEEP idle buffers and SCRATCH_BYTES in all stay per device; the
-// rest, and everything when the last weight of the device goes or an allocation fails, is given back to the driver.
+// device. Bounded: at most SCRATCH_KEEP idle buffers and SCRATCH_BYTES in all stay per device. The rest is given back to the
+// driver, and everything when the last weight of the device goes, when a model is built, when memory is short for a new
+// weight, and when an allocation of scratch or of a caller's buffer fails.
 constexpr size_t SCRATCH_KEEP = 6, SCRATCH_BYTES = size_t(256) << 20;
 struct Scratch {
     struct Buf { void* p; size_t bytes; };
@@ -61,7 +62,7 @@ struct Scratch {
         }
         for (const Buf& b : out) cudaFree(b.p);
     }
-    void release() {
+    bool release() {  // was there anything?
         std::vector<Buf> out;
         {
             std::lock_guard<std::mutex> lock(mu);
@@ -69,6 +70,16 @@ struct Scratch {
             idle_bytes = 0;
         }
         for (const Buf& b : out) cudaFree(b.p);
+        return !out.empty();
+    }
+    void make_room(size_t bytes) {  // on the current device: the idle buffers go when less than this is free
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (idle.empty()) return;
+        }
+        size_t free_bytes = 0, total = 0;
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) cudaGetLastError();
+        if (free_bytes < bytes) release();
     }
     void count(int d) {
         bool last = false;
@@ -152,10 +163,12 @@ int elb_device_count(void) {
 int elb_malloc(int device, size_t bytes, void** out) {
     if (!out) return fail(ELB_ERR_INVALID, "elb_malloc: null out");
     ELB_CUDA(cudaSetDevice(device));
-    if (cudaMalloc(out, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+    auto get = [&] {
+        if (cudaMalloc(out, std::max<size_t>(bytes, 16)) == cudaSuccess) return true;
         cudaGetLastError();
-        return fail(ELB_ERR_MEMORY, "elb_malloc: out of device memory");
-    }
+        return false;
+    };
+    if (!get() && !(scratch_of(device).release() && get())) return fail(ELB_ERR_MEMORY, "elb_malloc: out of device memory");
     return ELB_OK;
 }
 int elb_free(void* p) { ELB_CUDA(cudaFree(p)); return ELB_OK; }
@@ -186,6 +199,8 @@ int elb_device_sync(int device) {
 int elb_weight_create(int device, int ggml_type, int64_t rows, int64_t n, const void* bytes, size_t nbytes, int flags,
                       elb_weight** out) {
     if (elb_device_count() == 0) return fail(ELB_ERR_CUDA, std::string("no usable CUDA device: ") + g_error);
+    // (the raw bytes, the tiled ones, digit planes or fp16 pairs: up to four bytes a weight, on 4.5 bits)
+    if (cudaSetDevice(device) == cudaSuccess) scratch_of(device).make_room(12 * nbytes + (size_t(64) << 20));
     Weight* w = nullptr;
     ELB_TRY(weight_create(device, ggml_type, rows, n, bytes, nbytes, flags, &w));
     const int rc = gemv_prepare(w);
@@ -456,9 +471,13 @@ int elb_model_set_tensor(elb_model* m, int role, int layer, int ggml_type, int64
                          size_t nbytes) {
     return model_set_tensor(M(m), role, layer, ggml_type, rows, n, bytes, nbytes);
 }
-int elb_model_finalize(elb_model* m) { return model_finalize(M(m)); }
+int elb_model_finalize(elb_model* m) {
+    if (m) scratch_of(model_device(M(m))).release();
+    return model_finalize(M(m));
+}
 int elb_model_load_gguf(const char* path, int n_ctx, int device, int max_batch, int n_seq, elb_model** out) {
     if (!out) return fail(ELB_ERR_INVALID, "load_gguf: null argument");
+    scratch_of(device).release();
     Model* m = nullptr;
     ELB_TRY(model_load_gguf(path, n_ctx, device, max_batch, n_seq, 0, 1, nullptr, &m));  // the file is checked before any device is touched
     *out = reinterpret_cast<elb_model*>(m);
@@ -467,6 +486,7 @@ int elb_model_load_gguf(const char* path, int n_ctx, int device, int max_batch, 
 int elb_model_load_gguf_tp(const char* path, int n_ctx, int device, int max_batch, int n_seq, int tp_rank, int tp_size,
                            const void* id128, elb_model** out) {
     if (!out) return fail(ELB_ERR_INVALID, "load_gguf: null argument");
+    scratch_of(device).release();
     Model* m = nullptr;
     ELB_TRY(model_load_gguf(path, n_ctx, device, max_batch, n_seq, tp_rank, tp_size, id128, &m));
     *out = reinterpret_cast<elb_model*>(m);

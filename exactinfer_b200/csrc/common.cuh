@@ -399,6 +399,7 @@ int model_eval_batch_top(Model* m, int n, const int32_t* tokens, const int32_t* 
 int model_stats(const Model* m, float* ms, int64_t* launches);
 int model_hidden(Model* m, float* out);
 int model_fill_exchange(Model* m, int byte);
+int model_device(const Model* m);
 size_t model_weight_bytes(const Model* m);
 size_t model_kv_bytes_per_token(const Model* m);
 }  // namespace elb

@@ -80,6 +80,46 @@ def test_operator_scratch_of_a_failed_call_is_not_kept(elb):
     w.close()
 
 
+def test_idle_operator_scratch_gives_way(elb):
+    """Buffers, weights and models get the memory that lies idle in the operators' scratch."""
+    import ctypes as C
+    from exactinfer_b200 import capi
+
+    def free():
+        f, t = C.c_size_t(), C.c_size_t()
+        capi.check(capi.lib().elb_device_mem_info(0, C.byref(f), C.byref(t)))
+        return f.value
+
+    MB = 1 << 20
+    rng = np.random.default_rng(3)
+    w = elb.Weight(synth.Q8_0, 64, 4096, synth.rand_weight(rng, synth.Q8_0, 64, 4096), planes=True)
+    x = rng.normal(size=(8192, 4096)).astype(np.float32)
+    spec = synth.Spec(name="small", n_layer=1, n_embd=256, n_ff=512, n_head=2, n_head_kv=1, n_vocab=512, layout="q8_0")
+    tens = list(synth.generate(spec, 3))
+    big = synth.rand_weight(rng, synth.Q8_0, 1024, 16384)
+
+    def short_of_memory(left):  # the scratch holds 128 MB or more, about `left` MB are free beside it
+        w.matmul(x)
+        hold = C.c_void_p()
+        capi.check(capi.lib().elb_malloc(0, (free() - left * MB) // (2 * MB) * (2 * MB), C.byref(hold)))
+        assert free() < (left + 8) * MB
+        return hold
+
+    hold, buf = short_of_memory(40), C.c_void_p()
+    capi.check(capi.lib().elb_malloc(0, 100 * MB, C.byref(buf)))
+    for p in (buf, hold):
+        capi.check(capi.lib().elb_free(p))
+    hold = short_of_memory(40)
+    elb.Weight(synth.Q8_0, 1024, 16384, big, planes=True).close()  # 17 MB, tiled 17 MB, planes 16 MB or pairs 64 MB
+    capi.check(capi.lib().elb_free(hold))
+    hold = short_of_memory(240)
+    m = elb.Backend(spec, tens, 40000)  # 45 MB for the model's own count, and it wants 256 MB beside that
+    assert np.isfinite(m.eval(np.array([1], np.int32), 0)).all()
+    m.close()
+    capi.check(capi.lib().elb_free(hold))
+    w.close()
+
+
 # vocabularies below, at and just past a chunk of the reduction (2560 logits), and of several chunks
 @pytest.mark.parametrize("vocab", (64, 2559, 2560, 2561, 7681))
 def test_top_tokens_at_chunk_edges(elb, vocab):
