@@ -108,11 +108,12 @@ template <int GP, int KT> struct AcWarp {
 #pragma unroll
         for (int o = GP; o < 32; o *= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         const float m_new = fmaxf(m, mx);
-        const float p = on ? expf(score - m_new) : 0.f;
+        const float from = m_new == -INFINITY ? 0.f : m_new;  // (keys at -infinity: probability 0, also when no other has come yet)
+        const float p = on ? expf(score - from) : 0.f;
         float sum = p;
 #pragma unroll
         for (int o = GP; o < 32; o *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        const float corr = expf(m - m_new);  // (0 for the first tile)
+        const float corr = expf(m - from);  // (0 for the first tile)
         const bool moved = m_new != m;
         l = l * corr + sum;
         m = m_new;
@@ -165,7 +166,8 @@ __device__ __forceinline__ void ac_finish(const AcWarp<GP, KT>& w, const AcSmem&
             float M = -INFINITY;
 #pragma unroll
             for (int i = 0; i < WARPS; ++i) M = fmaxf(M, s.mw[i * 8 + h0 + lane]);
-            c = w.m == -INFINITY ? 0.f : expf(s.mw[warp * 8 + h0 + lane] - M);
+            const float mine = s.mw[warp * 8 + h0 + lane];
+            c = mine == -INFINITY ? 0.f : expf(mine - M);
             if (warp == 0) {
                 float L = 0.f;
 #pragma unroll

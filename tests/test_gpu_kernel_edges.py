@@ -230,6 +230,51 @@ def test_decode_long_and_short_contexts_in_turn(elb, n_layer):
     cpu.close()
 
 
+# keys whose score is -infinity for some query heads of a KV head and finite for the others: probability 0 for the former, the
+# latter as ever. The first keys, so that a warp's first tile has nothing else; alone in a tile; and behind finite ones.
+@pytest.mark.parametrize("special", ((0, 1, 2, 3), (0, 1, 2, 3, 4, 5, 6, 7, 8), (2,), (12, 13, 14, 15), (33, 34, 35, 36, 37, 38, 39)))
+def test_attention_scores_of_minus_infinity(elb, special):
+    spec = synth.Spec(name="small", n_layer=1, n_embd=256, n_ff=512, n_head=8, n_head_kv=1, n_vocab=512, layout="f16", head_sigma=2e-2)
+    rng, tens = np.random.default_rng(8), []
+    odd = 400  # the token of those keys: the only one with a value in column 7
+    for role, layer, t, rows, n, data in synth.generate(spec, 51):
+        if role in ("attn_q_norm", "attn_k_norm"):  # (dimension 63 is turned the least by the rotation)
+            data = data.copy().view(np.float32)
+            data[0, 63] = 1e10 if role == "attn_q_norm" else 1e30
+            data = data.view(np.uint8)
+        elif role in ("token_embd", "attn_q", "attn_k"):
+            w = data.copy().view(np.float16).reshape(rows, n)
+            if role == "token_embd":
+                w[:, 7] = 0
+                w[odd, 7] = 0.05
+                w[:, 3] = 0.05
+            elif role == "attn_k":  # k[63] > 0 for that token, 0 for the others
+                w[63] = 0
+                w[63, 7] = 0.1
+            else:                   # q[63] < 0 in heads 0..3; 0 there and in its partner of the rotation in heads 4..7
+                for h in range(8):
+                    w[h * 128 + 63] = w[h * 128 + 127] = 0
+                    w[h * 128 + 63, 3] = -0.1 if h < 4 else 0
+            data = w.view(np.uint8).reshape(rows, -1)
+        tens.append((role, layer, t, rows, n, data))
+    n_ctx = 100
+    toks = rng.integers(0, 399, n_ctx).astype(np.int32)
+    toks[list(special)] = odd
+    gpu, cpu = elb.Backend(spec, tens, n_ctx, n_seq=2), ol.OracleModel(spec, tens, n_ctx)
+    for s in (0, 1):
+        gpu.eval_batch(toks[:90], np.full(90, s), np.arange(90), want_logits=False)
+    cpu.eval(toks[:90], 0)
+    for pos in (45, 50, 59, 61, 89):
+        want = cpu.eval(toks[pos:pos + 1], pos)
+        assert np.isfinite(want).all()
+        one = gpu.eval(toks[pos:pos + 1], pos)
+        two = gpu.eval_batch(toks[[pos, pos]], [0, 1], [pos, pos])
+        for got in (one, two[0], two[1]):
+            assert np.abs(got - want).max() <= 2e-4 * np.abs(want).max(), pos
+    gpu.close()
+    cpu.close()
+
+
 # more query heads than the built-in shapes have, q and v in a costlier format than k: one thread block gets ten row tiles of k
 # alone, more than three times k's share by count
 def test_decode_uneven_cut_of_qkv(elb):
