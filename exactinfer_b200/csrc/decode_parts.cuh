@@ -57,8 +57,10 @@ __device__ __forceinline__ int sd_need(int type) { return type == ELB_Q4_K ? 1 :
 __device__ __forceinline__ int unit_bytes_of(int type) { return type == ELB_Q4_K ? Q4K_UNIT : type == ELB_Q6_K ? Q6K_UNIT : Q8_UNIT; }
 // 1 / sqrt(x) in double from the single-precision estimate and two Newton steps (relative error ~1e-27 of the exact
 // value before the last rounding): what the reference's 1.0 / sqrt(x) in double gives, after rounding to float,
-// without the division and square root routines
+// without the division and square root routines; those only beyond the range of a float (values of more than 1e19)
+static __device__ __noinline__ double rsqrt_far(double x) { return 1.0 / sqrt(x); }
 __device__ __forceinline__ double rsqrt_d(double x) {
+    if (!(x > 1e-37 && x < 1e38)) return rsqrt_far(x);
     double y = double(rsqrtf(float(x)));
     y = y * fma(-0.5 * x, y * y, 1.5);
     y = y * fma(-0.5 * x, y * y, 1.5);

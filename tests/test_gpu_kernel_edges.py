@@ -275,6 +275,26 @@ def test_attention_scores_of_minus_infinity(elb, special):
     cpu.close()
 
 
+# a residual stream whose mean square is beyond the range of a float: the norm's factor is taken in double, as the CPU path does
+@pytest.mark.parametrize("layout,factor", (("f16", 1e12), ("q8_0", 3e10), ("q4_k_m", 3e10)))
+def test_decode_with_a_very_large_residual_stream(elb, layout, factor):
+    spec = synth.Spec(name="small", n_layer=2, n_embd=256, n_ff=512, n_head=2, n_head_kv=1, n_vocab=512, layout=layout, head_sigma=2e-2)
+    tens = []
+    for role, layer, t, rows, n, data in synth.generate(spec, 53):
+        if role == "ffn_norm":
+            data = (data.copy().view(np.float32) * np.float32(factor)).view(np.uint8)
+        tens.append((role, layer, t, rows, n, data))
+    gpu, cpu = elb.Backend(spec, tens, 16), ol.OracleModel(spec, tens, 16)
+    toks = synth.lcg_tokens(8, spec.n_vocab, 53)
+    for pos in range(4):
+        a, b = gpu.eval(toks[pos:pos + 1], pos), cpu.eval(toks[pos:pos + 1], pos)
+        assert gpu.last_eval_stats()[1] == 1, "the persistent kernel must run"
+        assert np.square(gpu.hidden().astype(np.float64)).mean() > 1e39
+        assert np.abs(a - b).max() <= 2e-4 * np.abs(b).max() and np.abs(b).max() > 0
+    gpu.close()
+    cpu.close()
+
+
 # more query heads than the built-in shapes have, q and v in a costlier format than k: one thread block gets ten row tiles of k
 # alone, more than three times k's share by count
 def test_decode_uneven_cut_of_qkv(elb):
