@@ -22,8 +22,8 @@ namespace {
 // to the end of its scope. It goes back to the pool only from a call that has waited for all it enqueued (settled()), so
 // calls on other threads and streams never meet in one; a call that fails in between frees its buffers, which waits for the
 // device. Bounded: at most SCRATCH_KEEP idle buffers and SCRATCH_BYTES in all stay per device. The rest is given back to the
-// driver, and everything when the last weight of the device goes, when a model is built, when memory is short for a new
-// weight, and when an allocation of scratch or of a caller's buffer fails.
+// driver, and everything when the last weight of the device goes, when a model is built, and when an allocation of scratch,
+// of a weight or of a caller's buffer fails.
 constexpr size_t SCRATCH_KEEP = 6, SCRATCH_BYTES = size_t(256) << 20;
 struct Scratch {
     struct Buf { void* p; size_t bytes; };
@@ -72,15 +72,6 @@ struct Scratch {
         for (const Buf& b : out) cudaFree(b.p);
         return !out.empty();
     }
-    void make_room(size_t bytes) {  // on the current device: the idle buffers go when less than this is free
-        {
-            std::lock_guard<std::mutex> lock(mu);
-            if (idle.empty()) return;
-        }
-        size_t free_bytes = 0, total = 0;
-        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) cudaGetLastError();
-        if (free_bytes < bytes) release();
-    }
     void count(int d) {
         bool last = false;
         {
@@ -110,16 +101,7 @@ struct Dev {
         p = scratch_of(device).take(n, &bytes);
         if (p) return ELB_OK;
         bytes = n;
-        if (cudaMalloc(&p, n) != cudaSuccess) {
-            cudaGetLastError();
-            scratch_of(device).release();
-            if (cudaMalloc(&p, n) != cudaSuccess) {
-                cudaGetLastError();
-                p = nullptr;
-                return fail(ELB_ERR_MEMORY, "out of device memory");
-            }
-        }
-        return ELB_OK;
+        return device_malloc(&p, n) == cudaSuccess ? ELB_OK : fail(ELB_ERR_MEMORY, "out of device memory");
     }
     template <class T> T* as() const { return static_cast<T*>(p); }
 };
@@ -128,6 +110,20 @@ template <class... D> int settled(D&... d) {  // after the call's last wait
     return ELB_OK;
 }
 }  // namespace
+
+cudaError_t device_malloc_bytes(void** p, size_t bytes) {
+    int device = 0;
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) return e;
+    cudaGetLastError();
+    if (e == cudaErrorMemoryAllocation && cudaGetDevice(&device) == cudaSuccess && scratch_of(device).release()) {
+        e = cudaMalloc(p, bytes);
+        if (e == cudaSuccess) return e;
+        cudaGetLastError();
+    }
+    *p = nullptr;
+    return e;
+}
 }  // namespace elb
 
 using namespace elb;
@@ -163,12 +159,7 @@ int elb_device_count(void) {
 int elb_malloc(int device, size_t bytes, void** out) {
     if (!out) return fail(ELB_ERR_INVALID, "elb_malloc: null out");
     ELB_CUDA(cudaSetDevice(device));
-    auto get = [&] {
-        if (cudaMalloc(out, std::max<size_t>(bytes, 16)) == cudaSuccess) return true;
-        cudaGetLastError();
-        return false;
-    };
-    if (!get() && !(scratch_of(device).release() && get())) return fail(ELB_ERR_MEMORY, "elb_malloc: out of device memory");
+    if (device_malloc(out, std::max<size_t>(bytes, 16)) != cudaSuccess) return fail(ELB_ERR_MEMORY, "elb_malloc: out of device memory");
     return ELB_OK;
 }
 int elb_free(void* p) { ELB_CUDA(cudaFree(p)); return ELB_OK; }
@@ -199,8 +190,6 @@ int elb_device_sync(int device) {
 int elb_weight_create(int device, int ggml_type, int64_t rows, int64_t n, const void* bytes, size_t nbytes, int flags,
                       elb_weight** out) {
     if (elb_device_count() == 0) return fail(ELB_ERR_CUDA, std::string("no usable CUDA device: ") + g_error);
-    // (the raw bytes, the tiled ones, digit planes or fp16 pairs: up to four bytes a weight, on 4.5 bits)
-    if (cudaSetDevice(device) == cudaSuccess) scratch_of(device).make_room(12 * nbytes + (size_t(64) << 20));
     Weight* w = nullptr;
     ELB_TRY(weight_create(device, ggml_type, rows, n, bytes, nbytes, flags, &w));
     const int rc = gemv_prepare(w);

@@ -197,6 +197,10 @@ inline int launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem
 }
 
 // ---------------------------------------------------------------- host-side declarations shared between files
+// cudaMalloc on the current device; when memory is short the idle scratch of the operator calls goes first (capi.cu).
+// The error of an allocation that fails is cleared.
+cudaError_t device_malloc_bytes(void** p, size_t bytes);
+template <class T> inline cudaError_t device_malloc(T** p, size_t bytes) { return device_malloc_bytes(reinterpret_cast<void**>(p), bytes); }
 struct DeviceInfo {
     int sm_count = 0;
     size_t smem_optin = 0;

@@ -364,11 +364,11 @@ int gemv_prepare(Weight* w) {
     DeviceInfo di;
     ELB_TRY(device_info(w->device, &di));
     w->max_grid = di.sm_count * 2;
-    ELB_CUDA(cudaMalloc(&w->part, size_t(w->max_grid) * 2 * 16 * sizeof(float)));
-    ELB_CUDA(cudaMalloc(&w->counters, size_t(w->tiles) * sizeof(unsigned)));
+    ELB_CUDA(device_malloc(&w->part, size_t(w->max_grid) * 2 * 16 * sizeof(float)));
+    ELB_CUDA(device_malloc(&w->counters, size_t(w->tiles) * sizeof(unsigned)));
     ELB_CUDA(cudaMemset(w->counters, 0, size_t(w->tiles) * sizeof(unsigned)));
-    ELB_CUDA(cudaMalloc(&w->xlimbs, act_bytes(int(w->n))));
-    ELB_CUDA(cudaMalloc(&w->xinv, sizeof(float)));
+    ELB_CUDA(device_malloc(&w->xlimbs, act_bytes(int(w->n))));
+    ELB_CUDA(device_malloc(&w->xinv, sizeof(float)));
     return ELB_OK;
 }
 

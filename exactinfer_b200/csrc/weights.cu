@@ -166,8 +166,7 @@ int weight_create(int device, int type, int64_t rows_one, int64_t n, const void*
 
     uint8_t* raw = nullptr;
     auto cleanup = [&](int rc) { if (raw) cudaFree(raw); weight_destroy(w); return rc; };
-    if (cudaMalloc(&raw, nbytes) != cudaSuccess || cudaMalloc(&w->tiled, w->tiled_bytes) != cudaSuccess) {
-        cudaGetLastError();
+    if (device_malloc(&raw, nbytes) != cudaSuccess || device_malloc(&w->tiled, w->tiled_bytes) != cudaSuccess) {
         return cleanup(fail(ELB_ERR_MEMORY, "weight_create: out of device memory"));
     }
     if (cudaMemcpy(raw, bytes, nbytes, cudaMemcpyHostToDevice) != cudaSuccess)
@@ -191,8 +190,8 @@ int weight_create(int device, int type, int64_t rows_one, int64_t n, const void*
         static const bool off = [] { const char* v = std::getenv("ELB_Q8_PLANES"); return v && v[0] == '1'; }();
         const int64_t rows16 = w->tiles * 16;
         int* bad = nullptr;
-        if (!off && cudaMalloc(&bad, sizeof(int)) == cudaSuccess && cudaMemset(bad, 0, sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&w->f16pair, size_t(2) * rows16 * n * sizeof(__half)) == cudaSuccess) {
+        if (!off && device_malloc(&bad, sizeof(int)) == cudaSuccess && cudaMemset(bad, 0, sizeof(int)) == cudaSuccess &&
+            device_malloc(&w->f16pair, size_t(2) * rows16 * n * sizeof(__half)) == cudaSuccess) {
             const int64_t tot = rows16 * n;
             k_q8_pair<<<int(std::min<int64_t>((tot + 255) / 256, 148 * 32)), 256>>>(w->tiled, rows16, n, w->f16pair,
                                                                                    w->f16pair + rows16 * n, bad);
@@ -213,9 +212,9 @@ int weight_create(int device, int type, int64_t rows_one, int64_t n, const void*
         const int64_t rows16 = w->tiles * 16;
         w->n_planes = type == ELB_Q8_0 ? 1 : 2;
         const int blk = type == ELB_Q8_0 ? QK8_0 : QK_K;
-        bool ok = cudaMalloc(&w->planes, size_t(w->n_planes) * rows16 * n) == cudaSuccess &&
-                  cudaMalloc(&w->pl_d, size_t(rows16) * (n / blk) * sizeof(__half)) == cudaSuccess;
-        if (ok && type == ELB_Q4_K) ok = cudaMalloc(&w->pl_dm, size_t(rows16) * (n / 32) * sizeof(float)) == cudaSuccess;
+        bool ok = device_malloc(&w->planes, size_t(w->n_planes) * rows16 * n) == cudaSuccess &&
+                  device_malloc(&w->pl_d, size_t(rows16) * (n / blk) * sizeof(__half)) == cudaSuccess;
+        if (ok && type == ELB_Q4_K) ok = device_malloc(&w->pl_dm, size_t(rows16) * (n / 32) * sizeof(float)) == cudaSuccess;
         if (!ok) {
             cudaGetLastError();
             return cleanup(fail(ELB_ERR_MEMORY, "weight_create: out of device memory for the digit planes"));
