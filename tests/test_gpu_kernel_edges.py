@@ -175,11 +175,19 @@ def test_log_sum_exp_with_nan_and_infinity(elb, lo, hi, what):
     assert np.array_equal(ids, order) and np.array_equal(vals, full[order])
 
 
-def decode_pair(elb, spec, seed, n_ctx, walk):
+def runs_on(gpu, barrier_kernel=False):
+    """Which of the two persistent kernels a model's single steps run on (only the one-GPU kernel has exchange buffers)."""
+    from exactinfer_b200 import capi
+    rc = capi.lib().elb_selftest_decode_exchange(gpu._h, 0)
+    return rc == (capi.ERR_STATE if barrier_kernel else capi.OK)
+
+
+def decode_pair(elb, spec, seed, n_ctx, walk, barrier_kernel=False):
     """Single-token evaluations at the positions of `walk` (rows in front of them filled by prompt chunks), against the
     CPU oracle on the same cache contents; every evaluation twice, which must give the same bits."""
     tens = list(synth.generate(spec, seed))
     gpu, cpu = elb.Backend(spec, tens, n_ctx), ol.OracleModel(spec, tens, n_ctx)
+    assert runs_on(gpu, barrier_kernel)
     toks = synth.lcg_tokens(n_ctx, spec.n_vocab, seed)
     filled, worst = 0, 0.0
     for pos in walk:
@@ -204,6 +212,16 @@ def test_decode_across_attention_splits(elb, layout, heads, kv):
     spec = synth.Spec(name="small", n_layer=3, n_embd=512, n_ff=768, n_head=heads, n_head_kv=kv, n_vocab=1111, layout=layout,
                       head_sigma=2e-5)
     assert decode_pair(elb, spec, 31, 700, (0, 59, 60, 61, 650, 3, 651, 120)) <= 2e-4
+
+
+# the grid-barrier kernel, which tensor-parallel models run on, on one GPU: block formats, group sizes, split counts, a
+# feed-forward activation in global memory, and a cut of q|k|v that gives a thread block many more tiles of k than its share
+@pytest.mark.parametrize("layout,heads,kv,n_ff", (("q4_k_m", 8, 4, 768), ("q8_0", 8, 1, 768), ("q6_k", 2, 2, 768), ("q4_k_m", 2, 1, 25600)))
+def test_barrier_decode_kernel_on_one_gpu(elb, monkeypatch, layout, heads, kv, n_ff):
+    monkeypatch.setenv("ELB_DK_OLD", "1")
+    spec = synth.Spec(name="small", n_layer=3, n_embd=512, n_ff=n_ff, n_head=heads, n_head_kv=kv, n_vocab=1111, layout=layout,
+                      head_sigma=2e-5)
+    assert decode_pair(elb, spec, 33, 700, (0, 59, 60, 61, 650, 3, 651, 120), barrier_kernel=True) <= 2e-4
 
 
 # single evaluations at long and short contexts in turn, with an odd and an even number of short ones in between: what a step
@@ -297,7 +315,10 @@ def test_decode_with_a_very_large_residual_stream(elb, layout, factor):
 
 # more query heads than the built-in shapes have, q and v in a costlier format than k: one thread block gets ten row tiles of k
 # alone, more than three times k's share by count
-def test_decode_uneven_cut_of_qkv(elb):
+@pytest.mark.parametrize("barrier_kernel", (False, True))
+def test_decode_uneven_cut_of_qkv(elb, monkeypatch, barrier_kernel):
+    if barrier_kernel:
+        monkeypatch.setenv("ELB_DK_OLD", "1")
     spec = synth.Spec(name="small", n_layer=2, n_embd=512, n_ff=512, n_head=96, n_head_kv=12, n_vocab=512, layout="q4_k_m",
                       head_sigma=2e-5)
     tens = []
@@ -309,6 +330,7 @@ def test_decode_uneven_cut_of_qkv(elb):
         tens.append((role, layer, want, rows, n, data))
     toks = synth.lcg_tokens(150, spec.n_vocab, 37)
     gpu, cpu = elb.Backend(spec, tens, 160), ol.OracleModel(spec, tens, 160)
+    assert runs_on(gpu, barrier_kernel)
     gpu.eval(toks[:140], 0, want_logits=False)
     cpu.eval(toks[:140], 0)
     for pos in (0, 139, 140, 141):
