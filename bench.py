@@ -57,9 +57,9 @@ def micro_traffic():
 
 
 def decode_traffic(spec):
-    """DRAM bytes per k_decode_step launch, scaled per layer from the captures on 4 and 8 layers of the same shape
+    """DRAM bytes per k_decode_one launch (one GPU), scaled per layer from the captures on 4 and 8 layers of the same shape
     (fixed part for head and embedding row + a per-layer part, at positions ~517). None for shapes not captured."""
-    t = traffic_table().get("k_decode_step", {}).get(spec.name)
+    t = traffic_table().get("k_decode_one", {}).get(spec.name)
     return None if t is None else float(t["fixed_bytes"]) + float(t["per_layer_bytes"]) * spec.n_layer
 
 
@@ -640,10 +640,11 @@ def run_ours(args):
     per_step = launches / float(K)
     if per_step < 4:
         ach = step_bytes / step_s / 1e9
-        out["roofline"] = {"bound": "hbm", "kernel": "k_decode_step (one persistent launch per token: every matvec, "
-                           "norm, RoPE, attention and SwiGLU of the step)", "achieved": ach, "peak": hbm, "unit": "GB/s",
+        out["roofline"] = {"bound": "hbm", "kernel": ("k_decode_one" if world == 1 else "k_decode_step") + " (one persistent launch "
+                           "per token: every matvec, norm, RoPE, attention and SwiGLU of the step)", "achieved": ach, "peak": hbm, "unit": "GB/s",
                            "frac": ach / hbm, "peak_kind": peak_kind, "frac_of_8tbs": ach / 8000.0,
-                           "bytes_per_launch": step_bytes, "us_per_launch": step_s * 1e6, "traffic": decode_traffic(spec)}
+                           "bytes_per_launch": step_bytes, "us_per_launch": step_s * 1e6,
+                           "traffic": decode_traffic(spec) if world == 1 else None}
     if micro_ms is not None:
         ach = MICRO_BYTES / (micro_ms / 1000.0) / 1e9
         micro = {"bound": "hbm", "kernel": "k_gemv<Q4_K> 2560x9728, 4 limbs, alone (24 weight copies in rotation)",

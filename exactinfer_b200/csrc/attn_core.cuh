@@ -1,5 +1,5 @@
 // Attention of one query token over a range of cached keys, by all warps of a block (src/model.cpp:191-214 of the
-// reference): shared by the persistent decode kernel (decode.cu) and the batched rows kernel (attn.cu).
+// reference): shared by the one-GPU decode kernel (decode_one.cu) and the batched rows kernel (attn.cu).
 //
 // Bound by the bytes of the key and value rows, each read once for all query heads of its KV head, and at short contexts
 // by the chain of latencies: so every warp walks its own tiles of a few keys with its own running maximum, sum and

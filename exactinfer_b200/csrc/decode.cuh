@@ -74,7 +74,7 @@ struct DkParams {
     float* attn_part;       // [HKV][nsplit][group][130]
     unsigned* attn_counters;  // [HKV]
     unsigned* bar;          // grid barrier counter: counts arrivals for ever (compared modulo 2^32)
-    int* err;               // raised when a barrier wait ran out
+    int* err;               // raised when a bounded wait ran out
     int slots;              // row-tile slots per warp in the reduction buffer
     int cta_tiles;          // most row tiles a CTA's share of a matrix can touch
     int n_max;              // longest activation vector
@@ -97,7 +97,9 @@ struct DkParams {
 // q, k and v (p.kind[0 .. n_qkv), tiles and units set) share one phase: the CTAs cut the tiles of all together, by cost
 // (cost[i]: of a unit) or, with cost null, by count
 void decode_cut_qkv(DkParams& p, const long long* cost);
-// SM clocks of a unit of a block format on a working warp of decode.cu (measured there)
+// SM clocks that a unit of a block format takes a working warp when its weights have arrived (measured on decode.cu's 16 warps).
+// q|k|v of the built-in shapes is a few units per warp, which the rings hold when the stage starts. A long stream is bound by
+// HBM instead: on decode_one.cu gate|up of the 32B shape takes 0.86 us per Q4_K unit of a warp, 1.12 per Q6_K, 0.74 per Q8_0.
 inline long long decode_unit_cost(int type) { return type == ELB_Q6_K ? 1455 : type == ELB_Q8_0 ? 481 : 875; }
 
 // decode_one.cu (one GPU)

@@ -441,7 +441,7 @@ int chunk(Model* m, const int32_t* tokens, int B, int pos0, float* logits, const
         std::memcpy(top->ids, r + 8, size_t(top->k) * sizeof(int32_t));
         std::memcpy(top->vals, r + 8 + 4 * TOP_MAXK, size_t(top->k) * sizeof(float));
     }
-    if (m->err_host && *m->err_host) return fail(ELB_ERR_CUDA, "decode kernel: a grid barrier wait ran out");
+    if (m->err_host && *m->err_host) return fail(ELB_ERR_CUDA, "decode kernel: a bounded wait on another block or on weights ran out");
     if ((m->tpr && *m->tpr->err_host) || (m->tprows && *m->tprows->err_host))
         return fail(ELB_ERR_CUDA, "tensor parallel: a peer did not arrive at an all-reduce in time");
     ELB_TRY(gemm_tc_check());
@@ -1290,7 +1290,7 @@ int model_eval_steps(Model* m, const int32_t* tokens, int n, int pos0, float* de
     cudaFreeHost(pin);
     if (rc != ELB_OK) return rc;
     ELB_CUDA(e);
-    if (m->err_host && *m->err_host) return fail(ELB_ERR_CUDA, "decode kernel: a grid barrier wait ran out");
+    if (m->err_host && *m->err_host) return fail(ELB_ERR_CUDA, "decode kernel: a bounded wait on another block or on weights ran out");
     if ((m->tpr && *m->tpr->err_host) || (m->tprows && *m->tprows->err_host))
         return fail(ELB_ERR_CUDA, "tensor parallel: a peer did not arrive at an all-reduce in time");
     ELB_CUDA(cudaEventElapsedTime(device_ms, m->ev0, m->ev1));
