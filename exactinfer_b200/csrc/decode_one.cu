@@ -11,7 +11,7 @@
 //     going from exchange to exchange, every writer of exchange s of layer n + 1 has waited for (a CTA reads nothing in a
 //     stage in which it has no share, except the rows of the residual stream that its next share adds to). With the grid
 //     barriers of decode.cu (release, poll, then load: 2.5 us from the last store to the first use, against about 1 us) the
-//     4B-shape layer took 48.7 us, here 35.5 us. (Partial sums in 16-byte words of three values and the number, a quarter
+//     4B-shape layer took 48.7 us, here 34.7 us. (Partial sums in 16-byte words of three values and the number, a quarter
 //     fewer bytes: a step 2 % slower on the 0.6B and 1.7B shapes, 1 % faster on the 4B and 32B shapes. All vectors so: 5 %
 //     slower on the 0.6B and 4B shapes; two producers then share a 32-byte sector of the feed-forward vector.);
 //   * every working warp owns a fixed, contiguous share of the (row tile, k block) units of every weight matrix of the
